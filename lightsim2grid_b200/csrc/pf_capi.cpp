@@ -498,6 +498,7 @@ int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl,
     d.tfwd_phase = tiled ? I(otwp) : nullptr;
     d.tail_ct = P.tail_k > 0 ? P.tail_ct : P.m;
     d.tail_k = P.tail_k;
+    d.tail_w = 64;  // configure() widens it
     d.tail_map = P.tail_k > 0 ? I(otail) : nullptr;
     return 0;
 }
@@ -610,6 +611,13 @@ int configure(pf_plan *pl) {
     }
     const int lub = pl->precision ? 4 : 8, xb = pl->precision ? 4 : 8;
     const size_t static_smem = 2048;  // Shared struct of the kernel, rounded up
+    // the dense tail's staging area: all columns right of a panel when they fit beside the solve vector
+    // (an FP64 one: the mixed form's fallback uses the same width), else chunks of at least 64
+    if (P.tail_k > 0) {
+        pl->dp.tail_w = (P.tail_k + 31) & ~31;
+        while (pl->dp.tail_w > 64 && l2g::smem_bytes(pl->dp, 8, 8, false) + static_smem > (size_t)optin)
+            pl->dp.tail_w -= 32;
+    }
     size_t sm_in = l2g::smem_bytes(pl->dp, lub, xb, true);
     size_t sm_out = l2g::smem_bytes(pl->dp, lub, xb, false);
     bool fits = pl->dp.compact && sm_in + static_smem <= (size_t)optin;

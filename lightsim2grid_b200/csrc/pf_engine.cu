@@ -595,57 +595,234 @@ __device__ double voltage_update(const DevPlan &P, double2 *__restrict__ V, doub
 // that every row starts on 16 bytes).  After the factor program has applied the pivots before
 // the block (their updates of the block are the Schur complement of the sparse part),
 // tail_factor gathers the block from the LU and factorises it without pivoting, right-looking
-// in panels of tail_panel<LT>() columns: (a) the panel (rows [J, k)) staged in shared memory and
-// factorised there, one barrier per pivot; then, chunk after chunk of kTailChunk columns right of
-// the panel, (b) their U rows staged in shared memory (row stride kTailChunkLd) and solved there,
-// a warp per column and a lane per row, the pivots' values passed by shuffles (L of the panel's
-// diagonal block is unit lower) and (c) the trailing rows minus L U, each thread a register tile
-// of outputs read and written with 16-byte accesses.  Its pivots go back to the LU diagonal,
-// where the pivot scaling and the zero-pivot check read them.  Shared memory:
-// tail_smem_bytes(k) (the staging area also serves the substitutions' diagonal blocks).
-constexpr int kTailChunk = 128;
-// row stride of the staged U rows: rows start on 16 bytes, and the lanes of a warp reading one
-// column (a lane per row) fall in 8 different banks
-constexpr int kTailChunkLd = kTailChunk + 4;
+// in panels of NB = tail_panel<LT>() columns:
+// (a) the panel's diagonal block is factorised (a warp per row, a lane per column) and left in
+//     shared memory;
+// (b) every row below (its L values) and every column right of it (its U values) is an independent
+//     triangular solve against that block: a thread per row or column, its NB values in registers,
+//     the block's values by 16-byte broadcast reads; the results go to D and to shared memory
+//     (As by column of L, Bs by row of U);
+// (c) the trailing rows minus L U: each thread a register tile of TR x 4 outputs, 2 + 1 16-byte
+//     shared-memory reads per 32 multiply-adds (FP32), D read and written with 16-byte accesses.
+// With the whole panel factorised in shared memory, a barrier per pivot and 5 reads per 16
+// multiply-adds, the 391-step block took 1.64M SM cycles in FP32; now 0.93M: gather 145k, (a) 185k,
+// (b) 200k, (c) 400k (its multiply-adds alone: 156k).  2,848-bus grid with 300 chords, N-1: mixed
+// 72.8 -> 62.0 ms, FP64 131 -> 109 ms.
+// A right part wider than tail_w columns (the staging area's
+// share of shared memory) is solved and applied in chunks.  The block's pivots go back to the
+// LU diagonal, where the pivot scaling and the zero-pivot check read them.
 template <typename LT>
 __host__ __device__ constexpr int tail_panel() { return sizeof(LT) == 4 ? 32 : 16; }
 __host__ __device__ inline int tail_ld(int k) { return (k + 3) & ~3; }
-__host__ __device__ inline size_t tail_smem_bytes(int k, int lu_bytes) {
+__host__ __device__ inline int tail_lda(int k) { return (k + 7) & ~7; }
+// the diagonal block (TailPanel), As and a chunk of w columns of Bs
+__host__ __device__ inline size_t tail_smem_bytes(int k, int w, int lu_bytes) {
     const int nb = lu_bytes == 4 ? 32 : 16;
-    // the panel (k rows of nb + 1 values), then the chunk of U rows from a 16-byte boundary
-    return k > 0 ? ((((size_t)k * (nb + 1) + 3) & ~(size_t)3) + (size_t)nb * kTailChunkLd) * lu_bytes : 0;
+    return k > 0 ? (size_t)nb * (2 * nb + 1 + tail_lda(k) + w) * lu_bytes : 0;
 }
 
-// four consecutive values at a 16-byte boundary
-__device__ __forceinline__ void ld4(const float *p, float (&v)[4]) {
-    const float4 t = *reinterpret_cast<const float4 *>(p);
-    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-}
-__device__ __forceinline__ void ld4(const double *p, double (&v)[4]) {
-    const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void st4(float *p, const float (&v)[4]) {
-    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-__device__ __forceinline__ void st4(double *p, const double (&v)[4]) {
-    reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
-    reinterpret_cast<double2 *>(p)[1] = make_double2(v[2], v[3]);
-}
-
+// 16 bytes at a 16-byte boundary, in shared memory (an address of __cvta_generic_to_shared: the
+// functions below are not inlined, and a generic load costs more) or through a generic pointer
 template <typename LT>
-__device__ __noinline__ void tail_factor(const DevPlan &P, LT *lu, LT *D, LT *sm) {
+struct Vec16;
+template <>
+struct Vec16<float> {
+    static constexpr int N = 4;
+    static __device__ __forceinline__ void lds(unsigned a, float *v) {
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(a));
+    }
+    static __device__ __forceinline__ void sts(unsigned a, const float *v) {
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+    }
+    static __device__ __forceinline__ void ld(const float *p, float *v) {
+        const float4 t = *reinterpret_cast<const float4 *>(p);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    }
+    static __device__ __forceinline__ void st(float *p, const float *v) {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+};
+template <>
+struct Vec16<double> {
+    static constexpr int N = 2;
+    static __device__ __forceinline__ void lds(unsigned a, double *v) {
+        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(a));
+    }
+    static __device__ __forceinline__ void sts(unsigned a, const double *v) {
+        asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v[0]), "d"(v[1]) : "memory");
+    }
+    static __device__ __forceinline__ void ld(const double *p, double *v) {
+        const double2 t = *reinterpret_cast<const double2 *>(p);
+        v[0] = t.x; v[1] = t.y;
+    }
+    static __device__ __forceinline__ void st(double *p, const double *v) {
+        *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    }
+};
+__device__ __forceinline__ float lds(unsigned a, float v) {
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ double lds(unsigned a, double v) {
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts(unsigned a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts(unsigned a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
+
+// a / u from the pivot's reciprocal r: one product and one correction by the exact remainder
+// (Markstein, "IA-64 and Elementary Functions", ch. 8), which rounds as the quotient does, without its
+// branch on special operands
+__device__ __forceinline__ float tail_quotient(float a, float u, float r) {
+    const float q = a * r;
+    return fmaf(fmaf(-q, u, a), r, q);
+}
+__device__ __forceinline__ double tail_quotient(double a, double u, double r) {
+    const double q = a * r;
+    return fma(fma(-q, u, a), r, q);
+}
+
+// Shared memory of a panel: ush, row c = U(c, c ..) of the diagonal block from column 0, zero past its
+// end; lsh, row c = (0, L(c + 1, c), L(c + 2, c), ...), zero past its end; the reciprocal pivots.  So every step of (a) and (b) reads its NB values from the same place of the row, and
+// the solves are loops whose register arrays move down by one value a step: unrolled over all
+// steps (half the multiply-adds) the code of (a) and (b) did not stay in the instruction cache, and
+// the one warp of (a) took 34k cycles a panel, waiting for instructions.
+template <typename LT>
+struct TailPanel {
+    static constexpr int NB = tail_panel<LT>(), N = Vec16<LT>::N, E = (int)sizeof(LT);
+    static constexpr int kL = NB * NB * E, kR = 2 * NB * NB * E, kBytes = kR + NB * E;
+    // v[j - 1] = v[j] - f row[j] for j < W, row at shared address r
+    template <int W>
+    static __device__ __forceinline__ void step(LT (&v)[NB], unsigned r, LT f) {
+        LT u[W];
+#pragma unroll
+        for (int j = 0; j < W; j += N) Vec16<LT>::lds(r + j * E, u + j);
+#pragma unroll
+        for (int j = 1; j < W; ++j) v[j - 1] = v[j] - f * u[j];
+    }
+};
+
+// 1 / x for (a)'s serial chain.  FP32: the hardware's approximate reciprocal and one Newton step (the
+// quotient it serves corrects itself by the exact remainder).
+__device__ __forceinline__ float tail_reciprocal(float x) {
+    const float r = __fdividef(1.0f, x);
+    return fmaf(fmaf(-x, r, 1.0f), r, r);
+}
+__device__ __forceinline__ double tail_reciprocal(double x) { return 1.0 / x; }
+
+// (a) the diagonal block at row and column J (jb steps; past them the identity) to `sm` and back to D, by
+// the whole CTA: a warp per row (R rows each), a lane per column, the values in registers.  Per pivot:
+// its row from shared memory (`blk`, two rows used in turn), published by the row's warp after the
+// previous pivot, and one barrier; what (b) reads is written after the last one.  Bound by that serial
+// chain (read, shuffle, reciprocal, update, write, barrier): 322 cycles a pivot alone on an SM, against 620
+// with (b)'s rows written per pivot and 660 with the block in shared memory and a read-modify-write
+// per element; one warp with a row per lane took 758.
+template <typename LT, int R>
+__device__ __forceinline__ void tail_diagonal_rows(LT *D, int ld, int J, int jb, unsigned sm, unsigned blk) {
+    using T = TailPanel<LT>;
+    constexpr int NB = T::NB, E = T::E;
+    const int j = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    LT *base = D + (size_t)J * ld + J;
+    LT v[R];
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+        const int i = warp + s * nwarps;
+        v[s] = i < jb && j < jb ? base[(size_t)i * ld + j] : (LT)(i == j);
+    }
+    for (int e = threadIdx.x; e < 2 * NB * NB; e += blockDim.x) sts(sm + e * E, (LT)0);
+    if (warp == 0 && j < NB) sts(blk + j * E, v[0]);
+    __syncthreads();
+    for (int c = 0; c + 1 < NB; ++c) {
+        const unsigned row = blk + (c & 1) * NB * E, next = blk + ((c + 1) & 1) * NB * E;
+        const LT u = lds(row + (j < NB ? j : 0) * E, (LT)0), piv = __shfl_sync(0xffffffffu, u, c);
+        const LT r = tail_reciprocal(piv);
+#pragma unroll
+        for (int s = 0; s < R; ++s) {
+            const int i = warp + s * nwarps;
+            const LT f = tail_quotient(__shfl_sync(0xffffffffu, v[s], c), piv, r);
+            if (i > c) v[s] = j > c ? v[s] - f * u : (j == c ? f : v[s]);
+            if (i == c + 1 && j < NB) sts(next + j * E, v[s]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int s = 0; s < R; ++s) {
+        const int i = warp + s * nwarps;
+        if (i >= NB || j >= NB) continue;
+        sts(sm + (j >= i ? i * NB + j - i : NB * NB + j * NB + i - j) * E, v[s]);
+        if (i == j) sts(sm + T::kR + i * E, (LT)1 / v[s]);
+        if (i < jb && j < jb) base[(size_t)i * ld + j] = v[s];
+    }
+    __syncthreads();
+}
+template <typename LT>
+__device__ __noinline__ void tail_diagonal(LT *D, int ld, int J, int jb, unsigned sm, unsigned blk) {
     constexpr int NB = tail_panel<LT>();
-    constexpr int NP = NB + 1;  // panel row stride: the rows of one column fall in different banks
-    constexpr int TR = sizeof(LT) == 4 ? 4 : 2, TC = 4;  // register tile of the trailing update
-    const int k = P.tail_k, ld = tail_ld(k), tid = threadIdx.x, bd = blockDim.x;
-    const int kk = k * k;
-    // gather, four entries per thread in flight
-    for (int e0 = tid; e0 < kk; e0 += 4 * bd) {
+    const int nwarps = blockDim.x >> 5;
+    if (nwarps >= NB) tail_diagonal_rows<LT, 1>(D, ld, J, jb, sm, blk);
+    else if (nwarps * 2 >= NB) tail_diagonal_rows<LT, 2>(D, ld, J, jb, sm, blk);
+    else tail_diagonal_rows<LT, NB>(D, ld, J, jb, sm, blk);  // few warps: up to all rows each
+}
+
+// (b) one row below the diagonal block: L values (a full panel)
+template <typename LT>
+__device__ __forceinline__ void tail_row(LT *row, unsigned sm, unsigned as, int lda) {
+    using T = TailPanel<LT>;
+    constexpr int NB = T::NB, N = T::N, E = T::E;
+    LT a[NB];
+#pragma unroll
+    for (int j = 0; j < NB; j += N) Vec16<LT>::ld(row + j, a + j);
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll 1
+        for (int c = half * (NB / 2); c < (half + 1) * (NB / 2); c += N) {
+            LT rp[N], q[N];
+            Vec16<LT>::lds(sm + T::kR + c * E, rp);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const unsigned u = sm + (c + i) * NB * E;
+                q[i] = tail_quotient(a[0], lds(u, (LT)0), rp[i]);
+                sts(as + (unsigned)((c + i) * lda * E), q[i]);
+                if (half == 0) T::template step<NB>(a, u, q[i]);
+                else T::template step<NB / 2>(a, u, q[i]);
+            }
+            Vec16<LT>::st(row + c, q);
+        }
+}
+
+// (b) one column right of the diagonal block: U values (a full panel)
+template <typename LT>
+__device__ __forceinline__ void tail_column(LT *col, int ld, unsigned sm, unsigned bs, int ldb) {
+    using T = TailPanel<LT>;
+    constexpr int NB = T::NB, N = T::N, E = T::E;
+    LT v[NB];
+#pragma unroll
+    for (int r = 0; r < NB; ++r) v[r] = col[(size_t)r * ld];
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll 1
+        for (int c = half * (NB / 2); c < (half + 1) * (NB / 2); c += N)
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const LT u = v[0];
+                col[(size_t)(c + i) * ld] = u;
+                sts(bs + (unsigned)((c + i) * ldb * E), u);
+                if (half == 0) T::template step<NB>(v, sm + T::kL + (c + i) * NB * E, u);
+                else T::template step<NB / 2>(v, sm + T::kL + (c + i) * NB * E, u);
+            }
+}
+
+// The stages of tail_factor are functions of their own: inlined together they spilled inside
+// their loops.
+template <typename LT>
+__device__ __noinline__ void tail_gather(const int *__restrict__ map, const LT *lu, LT *D, int k) {
+    const int ld = tail_ld(k), bd = blockDim.x, kk = k * k;
+    // four entries per thread in flight
+    for (int e0 = threadIdx.x; e0 < kk; e0 += 4 * bd) {
         int p[4];
         LT v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) p[u] = e0 + u * bd < kk ? P.tail_map[e0 + u * bd] : -1;
+        for (int u = 0; u < 4; ++u) p[u] = e0 + u * bd < kk ? __ldg(map + e0 + u * bd) : -1;
 #pragma unroll
         for (int u = 0; u < 4; ++u) v[u] = p[u] >= 0 ? lu[p[u]] : (LT)0;
 #pragma unroll
@@ -655,92 +832,91 @@ __device__ __noinline__ void tail_factor(const DevPlan &P, LT *lu, LT *D, LT *sm
         }
     }
     __syncthreads();
-    LT *Ap = sm;                     // panel: Ap[(i - J) * NP + c], rows [J, k)
-    // U rows of the panel, one chunk: Bc[c * kTailChunkLd + q], from a 16-byte boundary (read with
-    // 16-byte loads; sm itself is 16-byte aligned)
-    LT *Bc = sm + (((size_t)k * NP + 3) & ~(size_t)3);
-    for (int J = 0; J < k; J += NB) {
-        const int jb = min(NB, k - J), J1 = J + jb, rows = k - J;
-        for (int e = tid; e < rows * NB; e += bd) {
-            const int i = e / NB, c = e - i * NB;
-            Ap[i * NP + c] = c < jb ? D[(size_t)(J + i) * ld + J + c] : (LT)0;
-        }
-        __syncthreads();
-        // (a) the panel, pivot after pivot
-        for (int c = 0; c < jb; ++c) {
-            const LT piv = Ap[c * NP + c];
-            for (int i = c + 1 + tid; i < rows; i += bd) {
-                LT *row = Ap + (size_t)i * NP;
-                const LT l = row[c] / piv;
-                row[c] = l;
-                for (int j = c + 1; j < jb; ++j) row[j] -= l * Ap[c * NP + j];
-            }
-            __syncthreads();
-        }
-        for (int e = tid; e < rows * NB; e += bd) {
-            const int i = e / NB, c = e - i * NB;
-            if (c < jb) D[(size_t)(J + i) * ld + J + c] = Ap[i * NP + c];
-        }
-        if (J1 >= k) break;
-        const int M = k - J1, tr = (M + TR - 1) / TR;
-        for (int j0 = J1; j0 < k; j0 += kTailChunk) {
-            const int w = min(kTailChunk, k - j0), tc = (w + TC - 1) / TC;
-            for (int e = tid; e < NB * kTailChunk; e += bd) {
-                const int c = e / kTailChunk, q = e - c * kTailChunk;
-                Bc[c * kTailChunkLd + q] = (c < jb && q < w) ? D[(size_t)(J + c) * ld + j0 + q] : (LT)0;
-            }
-            __syncthreads();
-            // (b) the chunk's U rows: a warp per column, lane i holds row i; at step c the lanes
-            // below c take row c's final value by a shuffle (the same updates in the same order
-            // as a sequential column solve)
-            {
-                const int lane = tid & 31, nwarps = bd >> 5;
-                for (int q = tid >> 5; q < w; q += nwarps) {
-                    LT v = lane < jb ? Bc[lane * kTailChunkLd + q] : (LT)0;
-                    for (int c = 0; c + 1 < jb; ++c) {
-                        const LT u = __shfl_sync(0xffffffffu, v, c);
-                        if (lane > c && lane < jb) v -= Ap[lane * NP + c] * u;
-                    }
-                    if (lane < jb) Bc[lane * kTailChunkLd + q] = v;
-                }
-            }
-            __syncthreads();
-            for (int e = tid; e < jb * kTailChunk; e += bd) {
-                const int c = e / kTailChunk, q = e - c * kTailChunk;
-                if (q < w) D[(size_t)(J + c) * ld + j0 + q] = Bc[c * kTailChunkLd + q];
-            }
-            // (c) the trailing rows: a tile of TR rows x 4 columns per thread (columns past the
-            // block's last fall in the row padding; their values are never read as entries)
-            for (int t = tid; t < tr * tc; t += bd) {
-                const int ti = t / tc, tj = t - ti * tc;
-                const int i0 = J1 + ti * TR, q0 = tj * TC;
-                LT acc[TR][TC];
+}
+
+// (b): `rows` rows below the diagonal block at (J, J) and the w columns from j0
+template <typename LT>
+__device__ __noinline__ void tail_solves(LT *D, int k, int J, int j0, int rows, int w, int W, unsigned sm) {
+    constexpr int NB = tail_panel<LT>(), E = (int)sizeof(LT);
+    const int ld = tail_ld(k), lda = tail_lda(k);
+    const unsigned as = sm + TailPanel<LT>::kBytes, bs = as + (unsigned)(NB * lda * E);
+    for (int t = threadIdx.x; t < rows + w; t += blockDim.x) {
+        if (t < rows)
+            tail_row<LT>(D + (size_t)(J + NB + t) * ld + J, sm, as + (unsigned)(t * E), lda);
+        else
+            tail_column<LT>(D + (size_t)J * ld + j0 + (t - rows), ld, sm, bs + (unsigned)((t - rows) * E), W);
+    }
+    __syncthreads();
+}
+
+// (c): rows and columns right of the panel (M rows from J1, w columns from j0) minus As Bs.  A warp per
+// 4 x 8 register tiles, a tile's columns in groups of 4 that are 32 apart (the lanes of a row read 128
+// consecutive bytes of Bs; columns past the block's last fall in the row padding, their values
+// are never read as entries).
+template <typename LT>
+__device__ __noinline__ void tail_update(LT *D, int k, int J1, int j0, int w, int W, unsigned sm) {
+    constexpr int NB = tail_panel<LT>(), N = Vec16<LT>::N, E = (int)sizeof(LT);
+    constexpr int TR = E == 4 ? 8 : 4, TG = 1;  // register tile: TR rows, TG groups of 4 columns
+    const int ld = tail_ld(k), lda = tail_lda(k), M = k - J1;
+    const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    const unsigned as = sm + TailPanel<LT>::kBytes, bs = as + (unsigned)(NB * lda * E);
+    const int sr = (M + 4 * TR - 1) / (4 * TR), sc = (w + 32 * TG - 1) / (32 * TG);
+    for (int t = threadIdx.x >> 5; t < sr * sc; t += nwarps) {
+        const int ti = t / sc, i0 = (ti * 4 + (lane >> 3)) * TR, q0 = (t - ti * sc) * 32 * TG + (lane & 7) * 4;
+        if (i0 >= M || q0 >= w) continue;
+        LT *C = D + (size_t)(J1 + i0) * ld + j0 + q0;
+        LT acc[TR][4 * TG];
 #pragma unroll
-                for (int r = 0; r < TR; ++r) {
-                    if (i0 + r < k) ld4(D + (size_t)(i0 + r) * ld + j0 + q0, acc[r]);
-                    else acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = (LT)0;
-                }
-                const LT *arow = Ap + (size_t)(i0 - J) * NP;
+        for (int r = 0; r < TR; ++r)
+#pragma unroll
+            for (int q = 0; q < 4 * TG; q += N) {
+                if (i0 + r < M && q0 + (q >> 2) * 32 < w)
+                    Vec16<LT>::ld(C + (size_t)r * ld + (q >> 2) * 32 + (q & 3), &acc[r][q]);
+                else
+#pragma unroll
+                    for (int i = 0; i < N; ++i) acc[r][q + i] = (LT)0;
+            }
+        const unsigned pa = as + (unsigned)(i0 * E), pb = bs + (unsigned)(q0 * E);
 #pragma unroll 4
-                for (int c = 0; c < NB; ++c) {
-                    LT a[TR], bq[TC];
+        for (int c = 0; c < NB; ++c) {
+            LT av[TR], bv[4 * TG];
 #pragma unroll
-                    for (int r = 0; r < TR; ++r) a[r] = i0 + r < k ? arow[r * NP + c] : (LT)0;
-                    ld4(Bc + c * kTailChunkLd + q0, bq);
+            for (int r = 0; r < TR; r += N) Vec16<LT>::lds(pa + (unsigned)((c * lda + r) * E), av + r);
 #pragma unroll
-                    for (int r = 0; r < TR; ++r)
+            for (int q = 0; q < 4 * TG; q += N)
+                Vec16<LT>::lds(pb + (unsigned)((c * W + (q >> 2) * 32 + (q & 3)) * E), bv + q);
 #pragma unroll
-                        for (int q = 0; q < TC; ++q) acc[r][q] -= a[r] * bq[q];
-                }
+            for (int r = 0; r < TR; ++r)
 #pragma unroll
-                for (int r = 0; r < TR; ++r)
-                    if (i0 + r < k) st4(D + (size_t)(i0 + r) * ld + j0 + q0, acc[r]);
-            }
-            __syncthreads();
+                for (int q = 0; q < 4 * TG; ++q) acc[r][q] -= av[r] * bv[q];
+        }
+#pragma unroll
+        for (int r = 0; r < TR; ++r)
+#pragma unroll
+            for (int q = 0; q < 4 * TG; q += N)
+                if (i0 + r < M && q0 + (q >> 2) * 32 < w)
+                    Vec16<LT>::st(C + (size_t)r * ld + (q >> 2) * 32 + (q & 3), &acc[r][q]);
+    }
+    __syncthreads();
+}
+
+template <typename LT>
+__device__ __noinline__ void tail_factor(const DevPlan &P, LT *lu, LT *D, LT *smem) {
+    constexpr int NB = tail_panel<LT>();
+    const int k = P.tail_k, ld = tail_ld(k), W = P.tail_w;
+    tail_gather<LT>(P.tail_map, lu, D, k);
+    const unsigned sm = (unsigned)__cvta_generic_to_shared(smem);
+    for (int J = 0; J < k; J += NB) {
+        const int jb = min(NB, k - J), J1 = J + jb, M = k - J1;
+        tail_diagonal<LT>(D, ld, J, jb, sm, sm + TailPanel<LT>::kBytes);  // As is not in use yet
+        for (int j0 = J1; j0 < k; j0 += W) {
+            const int w = min(W, k - j0);
+            tail_solves<LT>(D, k, J, j0, j0 == J1 ? M : 0, w, W, sm);
+            tail_update<LT>(D, k, J1, j0, w, W, sm);
         }
     }
     __syncthreads();
-    for (int c = tid; c < k; c += bd) lu[P.dpos[P.tail_ct + c]] = D[(size_t)c * ld + c];
+    for (int c = threadIdx.x; c < k; c += blockDim.x) lu[P.dpos[P.tail_ct + c]] = D[(size_t)c * ld + c];
     __syncthreads();
 }
 
@@ -771,7 +947,14 @@ __device__ __noinline__ void tail_forward(const DevPlan &P, const LT *D, XT *x, 
         for (int i = J1 + tid; i < k; i += bd) {
             XT v = xt[i];
             const LT *row = D + (size_t)i * ld + J;
-            for (int c = 0; c < jb; ++c) v -= (XT)row[c] * xt[J + c];
+            // the panel is full here (rows below it exist): 16-byte reads of the row
+#pragma unroll
+            for (int c = 0; c < 32; c += Vec16<LT>::N) {
+                LT r[Vec16<LT>::N];
+                Vec16<LT>::ld(row + c, r);
+#pragma unroll
+                for (int u = 0; u < Vec16<LT>::N; ++u) v -= (XT)r[u] * xt[J + c + u];
+            }
             xt[i] = v;
         }
         __syncthreads();
@@ -809,7 +992,17 @@ __device__ __noinline__ void tail_backward(const DevPlan &P, Shared &S, const LT
         for (int i = tid; i < J; i += bd) {
             XT v = xt[i];
             const LT *row = D + (size_t)i * ld + J;
-            for (int c = 0; c < jb; ++c) v -= (XT)row[c] * (XT)S.red[c];
+            if (jb == 32) {
+#pragma unroll
+                for (int c = 0; c < 32; c += Vec16<LT>::N) {
+                    LT r[Vec16<LT>::N];
+                    Vec16<LT>::ld(row + c, r);
+#pragma unroll
+                    for (int u = 0; u < Vec16<LT>::N; ++u) v -= (XT)r[u] * (XT)S.red[c + u];
+                }
+            } else {
+                for (int c = 0; c < jb; ++c) v -= (XT)row[c] * (XT)S.red[c];
+            }
             xt[i] = v;
         }
         __syncthreads();
@@ -1723,7 +1916,7 @@ size_t smem_bytes(const DevPlan &P, int lu_bytes, int x_bytes, bool lu_in_smem) 
     const size_t nb = P.nar_off[3] > 0 ? (((xb + lb + bb + 7) & ~(size_t)7) - (xb + lb + bb)) + (size_t)P.nar_off[3] * 8 : 0;
     // the dense tail's staging area, 16-byte aligned after the tables (global-memory LU)
     if (!lu_in_smem && P.tail_k > 0)
-        return ((xb + lb + bb + nb + 7) & ~(size_t)7) + 16 + tail_smem_bytes(P.tail_k, lu_bytes);
+        return ((xb + lb + bb + nb + 7) & ~(size_t)7) + 16 + tail_smem_bytes(P.tail_k, P.tail_w, lu_bytes);
     return xb + lb + bb + nb;
 }
 

@@ -50,6 +50,7 @@ struct DevPlan {
     // substituted as one dense row-major block in the CTA's slab; tail_map: LU position of each
     // block entry (-1 outside the pattern)
     int tail_ct, tail_k;
+    int tail_w;              // columns of U that its staging area holds (a multiple of 32)
     const int *tail_map;
 };
 

@@ -95,3 +95,42 @@ def test_dense_tail_single_pf_matches_oracle(precision):
         if precision == 0:
             assert s.get_nb_iter() == o.get_nb_iter(), name
         assert _vdiff(s.get_V(), o.get_V()) <= (TOL_FP64 if precision == 0 else TOL_MIXED), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,threads", [(0, 64), (0, 256), (0, 512), (1, 64), (1, 512), (1, 768)])
+def test_dense_tail_thread_counts(precision, threads):
+    """The diagonal block's rows per warp depend on the CTA's warps (1, 2 or up to all of them)."""
+    from lightsim2grid_b200 import Plan
+
+    c = grid_problem("grid2848c300")
+    o = OracleNR(False)
+    assert o.compute_pf(c["Ybus"], c["V0"], c["Sbus"], c["ref"], c["weights"], c["pv"], c["pq"], 10, 1e-8)
+    plan = Plan(c["Ybus"], c["V0"], c["Sbus"], c["ref"], c["weights"], c["pv"], c["pq"], precision=precision,
+                threads=threads)
+    assert plan.info()["tail_k"] % 16 != 0  # the last panel is partial in both precisions
+    V, conv, it, err = plan.solve(c["V0"], c["Sbus"], 10, 1e-8)
+    assert conv
+    assert _vdiff(V, o.get_V()) <= (TOL_FP64 if precision == 0 else TOL_MIXED)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1])
+def test_dense_tail_in_column_chunks(precision):
+    """A block whose right part does not fit beside the solve vector is solved in column chunks:
+    FP64 solve vector 95 KB, 594 steps, 16 x (33 + 600 + 608) x 8 = 159 KB over 227 KB together."""
+    from lightsim2grid_b200 import Plan, synthetic
+
+    g, V0 = synthetic.make_grid(6515, 8796, 1100, seed=6516, chords=350)
+    Y, S = g.get_Ybus(), g.get_Sbus()
+    args = (g.get_slack_ids(), g.get_slack_weights(), g.get_pv(), g.get_pq())
+    S2 = S * 1.01
+    o = OracleNR(False)
+    assert o.compute_pf(Y, V0, S2, *args, 10, 1e-8)
+    plan = Plan(Y, V0, S, *args, precision=precision)
+    assert plan.info()["tail_k"] > 500
+    V, conv, it, err = plan.solve(V0, S2, 10, 1e-8)
+    assert conv
+    if precision == 0:
+        assert it == o.get_nb_iter()
+    assert _vdiff(V, o.get_V()) <= (TOL_FP64 if precision == 0 else TOL_MIXED)
