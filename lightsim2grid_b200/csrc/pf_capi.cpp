@@ -27,6 +27,9 @@ namespace {
 
 thread_local std::string g_err;
 
+// static shared memory of the Newton and DC kernels (Shared, Segment, the loop's job), rounded up
+constexpr size_t kNrStaticSmem = 2304;
+
 int fail(int code, const std::string &msg) {
     g_err = msg;
     return code;
@@ -182,7 +185,7 @@ struct pf_plan {
     int tile_ones = 0;       // instances for which tile_aux holds the row of ones
     bool last_tile = false;  // the last launch ran the batch-interleaved kernel
     // device work buffers
-    DevBuf scratch, counter, V0, Sbus, optr, opos, oval, jfirst, jcount, Vout, iters, errs, Jout, cycles, Vcase,
+    DevBuf scratch, counter, V0, Sbus, optr, opos, oval, jfirst, jcount, Vout, iters, errs, Jout, Vlast, cycles, Vcase,
         casemap;
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;  // result downloads that overlap the FP64 re-run
@@ -373,6 +376,73 @@ std::vector<int> pack_pairs(const std::vector<int> &a, const std::vector<int> &b
     return out;
 }
 
+// The Ybus rows by slots (DevPlan::row_*, off_*, dg_*): host arrays of one plan.
+struct RowSlots {
+    int slots = 0, len = 0;
+    std::vector<int> bus, slice, col, pos, target, x, dpos, dtarget, deq, dx, of_csr;
+};
+
+void build_row_slots(const l2g::Plan &P, RowSlots &R) {
+    const int n = P.n;
+    std::vector<int> deg(n, 0), order(n);
+    for (int r = 0; r < n; ++r) {
+        order[r] = r;
+        for (int p = P.Rp[r]; p < P.Rp[r + 1]; ++p) deg[r] += P.Rj[p] != r;
+    }
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return deg[a] > deg[b]; });
+    const int ns = (n + 31) / 32;
+    R.slots = ns * 32;
+    R.bus.assign(R.slots, -1);
+    R.slice.resize(2 * (size_t)ns);
+    R.dpos.assign(R.slots, -1);
+    R.dtarget.assign(4 * (size_t)R.slots, -1);
+    R.deq.assign(2 * (size_t)R.slots, -1);
+    R.dx.assign(2 * (size_t)R.slots, -1);
+    R.of_csr.assign(P.nnzY, 0);
+    for (int g = 0, at = 0; g < ns; ++g) {
+        const int width = deg[order[32 * (size_t)g]];  // the slice's longest row comes first
+        R.slice[2 * g] = at;
+        R.slice[2 * g + 1] = width;
+        at += 32 * width;
+        R.len = at;
+    }
+    R.col.assign(R.len, -1);
+    R.pos.assign(R.len, -1);
+    R.target.assign(4 * (size_t)R.len, -1);
+    R.x.assign(2 * (size_t)R.len, -1);
+    const bool newton = !P.ytarget.empty();
+    for (int s = 0; s < n; ++s) {
+        const int r = order[s];
+        R.bus[s] = r;
+        if (!P.xP.empty()) {
+            R.deq[2 * s] = P.xP[r];
+            R.deq[2 * s + 1] = P.xQ[r];
+            R.dx[2 * s] = P.xVa[r];
+            R.dx[2 * s + 1] = P.xVm[r];
+        }
+        int at = R.slice[2 * (s / 32)] + s % 32;
+        for (int p = P.Rp[r]; p < P.Rp[r + 1]; ++p) {
+            const int c = P.Rj[p];
+            const bool diag = c == r;
+            int *t = diag ? &R.dtarget[4 * (size_t)s] : &R.target[4 * (size_t)at];
+            if (newton) std::copy(&P.ytarget[4 * (size_t)p], &P.ytarget[4 * (size_t)p] + 4, t);
+            if (diag) {
+                R.dpos[s] = p;
+                R.of_csr[p] = -1 - s;
+                continue;
+            }
+            R.col[at] = c;
+            R.pos[at] = p;
+            R.of_csr[p] = at;
+            if (!P.xP.empty()) {
+                R.x[2 * (size_t)at] = P.xVa[c];
+                R.x[2 * (size_t)at + 1] = P.xVm[c];
+            }
+            at += 32;
+        }
+    }
+}
+
 // Uploads the structure arrays of one plan (and, for a fast-decoupled system, its factor
 // values) into two device blobs and points the fields of `d` into them.
 int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl, const std::vector<double> *luval,
@@ -425,6 +495,19 @@ int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl,
             if (r == P.slack0) wJ[r] = P.weights[r];
             else if (std::fabs(P.weights[r]) > 1e-7) wJ[r] = P.weights[r];
         }
+    // the row slots of the Newton and fast-decoupled kernels' Ybus passes
+    RowSlots R;
+    if (!P.dc && P.nnzY > 0) build_row_slots(P, R);
+    std::vector<double> off(2 * (size_t)R.len, 0.0), dg(2 * (size_t)R.slots, 0.0);
+    for (int p = 0; p < (int)R.of_csr.size(); ++p) {
+        double *v = R.of_csr[p] >= 0 ? &off[2 * (size_t)R.of_csr[p]] : &dg[2 * (size_t)(-1 - R.of_csr[p])];
+        v[0] = rx[2 * (size_t)p];
+        v[1] = rx[2 * (size_t)p + 1];
+    }
+    size_t orb = push(bi, R.bus), ors = push(bi, R.slice), orc = push(bi, R.col), orp = push(bi, R.pos);
+    size_t ort = push(bi, R.target), orx = push(bi, R.x), odp = push(bi, R.dpos), odt = push(bi, R.dtarget);
+    size_t ode = push(bi, R.deq), odx = push(bi, R.dx), ocr = push(bi, R.of_csr);
+    size_t oov = push(bd, off), odv = push(bd, dg);
     size_t oRx = push(bd, rx), ow = push(bd, P.weights), ocv = push(bd, P.cval), owJ = push(bd, wJ);
     size_t olu = push(bd, luval ? *luval : std::vector<double>());
     if (d_int) cudaFree(d_int);
@@ -452,6 +535,22 @@ int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl,
     d.Rj = I(oRj);
     d.Rrow = I(oRrow);
     d.Rx = reinterpret_cast<const double2 *>(D(oRx));
+    auto I2 = [&](size_t o) { return reinterpret_cast<const int2 *>(bI + o); };
+    d.row_slots = R.slots;
+    d.row_len = R.len;
+    d.row_bus = I(orb);
+    d.row_slice = I2(ors);
+    d.off_col = I(orc);
+    d.off_pos = I(orp);
+    d.off_val = reinterpret_cast<const double2 *>(D(oov));
+    d.off_target = I4(ort);
+    d.off_x = I2(orx);
+    d.dg_pos = I(odp);
+    d.dg_val = reinterpret_cast<const double2 *>(D(odv));
+    d.dg_target = I4(odt);
+    d.dg_eq = I2(ode);
+    d.dg_x = I2(odx);
+    d.row_of_csr = I(ocr);
     d.w = D(ow);
     d.ytarget = I4(oyt);
     d.yjpos = I4(oyj);
@@ -610,7 +709,7 @@ int configure(pf_plan *pl) {
         return 0;
     }
     const int lub = pl->precision ? 4 : 8, xb = pl->precision ? 4 : 8;
-    const size_t static_smem = 2048;  // Shared struct of the kernel, rounded up
+    const size_t static_smem = kNrStaticSmem;
     // the dense tail's staging area: all columns right of a panel when they fit beside the solve vector
     // (an FP64 one: the mixed form's fallback uses the same width), else chunks of at least 64
     if (P.tail_k > 0) {
@@ -662,7 +761,7 @@ int configure(pf_plan *pl) {
 
 void release(pf_plan *pl) {
     for (DevBuf *b : {&pl->tile_scratch, &pl->tile_aux, &pl->scratch, &pl->counter, &pl->V0, &pl->Sbus, &pl->optr, &pl->opos, &pl->oval,
-                      &pl->jfirst, &pl->jcount, &pl->Vout, &pl->iters, &pl->errs, &pl->Jout, &pl->cycles,
+                      &pl->jfirst, &pl->jcount, &pl->Vout, &pl->iters, &pl->errs, &pl->Jout, &pl->Vlast, &pl->cycles,
                       &pl->Vcase, &pl->casemap})
         b->release();
     if (pl->d_int) cudaFree(pl->d_int);
@@ -696,7 +795,7 @@ void release(pf_plan *pl) {
 constexpr int kAutoTileLU = 60000;
 
 bool use_tile(const pf_plan *pl, const l2g::BatchArgs &a) {
-    if (pl->P.dc || pl->P.fdpf || a.chain || a.Jout || a.trace || a.reuse_below > 0) return false;
+    if (pl->P.dc || pl->P.fdpf || a.chain || a.Vlast || a.trace || a.reuse_below > 0) return false;
     if (pl->P.tail_k > 0) return false;  // the dense tail runs in the one-CTA kernel
     if (pl->opt.batch_layout == 2) return true;
     return pl->opt.batch_layout == 0 && !pl->lu_in_smem && pl->P.nnzLU >= kAutoTileLU && a.njobs >= 4 * pl->num_sms;
@@ -828,7 +927,7 @@ int launch_into(pf_plan *pl, l2g::BatchArgs a, int precision, cudaStream_t st, u
         size_t slab = l2g::slab_bytes(pl->dp, lub, in);
         int optin = 0;
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, pl->device);
-        if (in && (need + 2048 > (size_t)optin || !pl->dp.compact)) {
+        if (in && (need + kNrStaticSmem > (size_t)optin || !pl->dp.compact)) {
             in = false;
             need = l2g::smem_bytes(pl->dp, lub, lub, false);
             slab = l2g::slab_bytes(pl->dp, lub, false);
@@ -896,7 +995,9 @@ int run_batch(pf_plan *pl, int n_inst, const cplx *V0, long long v0_stride, cons
         return cuda_fail(e, "batch: alloc");
     if ((e = pl->iters.ensure((size_t)n_inst * sizeof(int))) != cudaSuccess) return cuda_fail(e, "batch: alloc");
     if ((e = pl->errs.ensure((size_t)n_inst * sizeof(int))) != cudaSuccess) return cuda_fail(e, "batch: alloc");
-    if (want_J && (e = pl->Jout.ensure(pl->P.Ji.size() * sizeof(double))) != cudaSuccess)
+    want_J = want_J && !pl->P.dc && !pl->P.fdpf;  // those have no Jacobian
+    if (want_J && ((e = pl->Jout.ensure(pl->P.Ji.size() * sizeof(double))) != cudaSuccess ||
+                   (e = pl->Vlast.ensure((size_t)n * sizeof(cplx))) != cudaSuccess))
         return cuda_fail(e, "batch: alloc");
     double t1 = now();
     l2g::BatchArgs a{};
@@ -921,10 +1022,18 @@ int run_batch(pf_plan *pl, int n_inst, const cplx *V0, long long v0_stride, cons
     }
     a.iters = static_cast<int *>(pl->iters.p);
     a.errs = static_cast<int *>(pl->errs.p);
-    a.Jout = want_J ? static_cast<double *>(pl->Jout.p) : nullptr;
+    a.Vlast = want_J ? static_cast<double2 *>(pl->Vlast.p) : nullptr;
     a.j_inst = 0;
     cudaEventRecord(pl->ev0, st);
+    // the Jacobian values of the last Newton step follow the launch in the stream
+    const auto jacobian = [&]() -> int {
+        if (!want_J) return 0;
+        const cudaError_t je = l2g::launch_jacobian_values(pl->dp, static_cast<const double2 *>(pl->Vlast.p),
+                                                           static_cast<double *>(pl->Jout.p), pl->num_sms, st);
+        return je == cudaSuccess ? 0 : cuda_fail(je, "batch: Jacobian values");
+    };
     int rc = launch(pl, a, pl->precision, st);
+    if (!rc) rc = jacobian();
     if (rc) return rc;
     cudaEventRecord(pl->ev1, st);
     // host work that overlaps the kernel (before any copy that would wait for it)
@@ -971,6 +1080,7 @@ int run_batch(pf_plan *pl, int n_inst, const cplx *V0, long long v0_stride, cons
             a.njobs = (int)rf.size();
             cudaEventRecord(pl->ev0, st);
             rc = launch(pl, a, 0, st);
+            if (!rc) rc = jacobian();
             if (rc) return rc;
             cudaEventRecord(pl->ev1, st);
             if (settled && (rc = (*settled)(again)) != 0) return rc;
@@ -1031,7 +1141,7 @@ BatchArgs device_args(const pf_device_batch *b) {
     a.Vout = static_cast<double2 *>(b->Vout);
     a.iters = b->iters;
     a.errs = b->errs;
-    a.Jout = nullptr;
+    a.Vlast = nullptr;
     a.j_inst = -1;
     return a;
 }
@@ -1358,6 +1468,8 @@ int pf_set_ybus_values(pf_plan *pl, const double *ybus_ri) {
     }
     cudaError_t e = cudaMemcpy(const_cast<double2 *>(pl->dp.Rx), rx.data(), rx.size() * sizeof(double),
                                cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = l2g::launch_set_ybus(pl->dp, pl->dp.Rx, pl->num_sms, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) return cuda_fail(e, "pf_set_ybus_values");
     compute_bridges(pl);
     return 0;
@@ -2332,8 +2444,8 @@ int pf_assemble_ybus_device(int nnz, const int *cptr, const int *cids, const dou
 
 int pf_set_ybus_values_device(pf_plan *pl, const double *ybus_ri, void *stream) {
     if (!pl || !ybus_ri) return fail(-1, "pf_set_ybus_values_device: null argument");
-    cudaError_t e = cudaMemcpyAsync(const_cast<double2 *>(pl->dp.Rx), ybus_ri, (size_t)pl->P.nnzY * 16,
-                                    cudaMemcpyDeviceToDevice, static_cast<cudaStream_t>(stream));
+    cudaError_t e = l2g::launch_set_ybus(pl->dp, reinterpret_cast<const double2 *>(ybus_ri), pl->num_sms,
+                                         static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? 0 : cuda_fail(e, "pf_set_ybus_values_device");
 }
 

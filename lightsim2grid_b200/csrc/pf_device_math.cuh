@@ -15,25 +15,23 @@ __device__ __forceinline__ double cabs2(double2 a) { return sqrt(a.x * a.x + a.y
 
 constexpr double kPi = 3.141592653589793;
 
-// dS/dVa and dS/dVm of Ybus entry (r, c), as BaseNRAlgo::_dSbus_dV (BaseNRAlgo.tpp:228-257)
-__device__ __forceinline__ void dsbus(double2 y, double2 vr, double2 vc, bool diag, double2 ib, double &dvar,
-                                      double &dvai, double2 &dvm) {
-    const double ic = 1.0 / cabs2(vc);
-    const double2 vnc = make_double2(vc.x * ic, vc.y * ic);
-    double2 a = cmul(cconj(cmul(y, vnc)), vr);  // conj(Y * Vnorm_c) * V_r
-    double2 b = cmul(y, vc);                    // Y * V_c
-    if (diag) {
-        const double ir = 1.0 / cabs2(vr);
-        const double2 vnr = make_double2(vr.x * ir, vr.y * ir);
-        const double2 t = cmul(cconj(ib), vnr);
-        a.x += t.x;
-        a.y += t.y;
-        b.x -= ib.x;
-        b.y -= ib.y;
-    }
-    dvar = b.x * vr.y - b.y * vr.x;  // conj(-b) * (j V_r)
-    dvai = -(b.x * vr.x + b.y * vr.y);
-    dvm = a;
+// t = conj(y V_c) V_r of a Ybus entry (r, c) from b = y V_c: its complex power at the row.  A zero
+// V_c has no dS/d|V|: t becomes NaN, so that the step ends the instance with InifiniteValue.
+__device__ __forceinline__ double2 entry_power(double2 b, double2 vc, double2 vr) {
+    const int any = ((__double2hiint(vc.x) | __double2hiint(vc.y)) << 1) | __double2loint(vc.x) | __double2loint(vc.y);
+    const double2 t = cmul(cconj(b), vr);
+    return any != 0 ? t : make_double2(nan(""), nan(""));
+}
+
+// Jacobian values of Ybus entry (r, c) from t = conj(y V_c) V_r: dS/dVa = -j (t - d) and
+// |V_c| dS/d|V_c| = t + d, with d = conj(I_r) V_r on the diagonal, else 0 (the dS/dVa and dS/dVm of
+// BaseNRAlgo::_dSbus_dV, BaseNRAlgo.tpp:228-257, the latter's column c times |V_c|: the Newton
+// unknown is dVm / |V|, which the voltage update multiplies by |V|).  The scaled columns need no
+// |V| and no quotient: two complex products per entry in place of three, a square root and a division.
+__device__ __forceinline__ void dsbus(double2 t, double2 d, double &dvar, double &dvai, double2 &dvm) {
+    dvar = t.y - d.y;
+    dvai = d.x - t.x;
+    dvm = make_double2(t.x + d.x, t.y + d.y);
 }
 
 // a / b: correctly rounded in FP64; in FP32 (mixed form) the reciprocal-based quotient

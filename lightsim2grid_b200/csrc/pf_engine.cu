@@ -20,6 +20,7 @@
 #include "pf_engine.cuh"
 #include "pf_device_math.cuh"
 
+#include <algorithm>
 #include <mutex>
 #include <set>
 #include <utility>
@@ -36,6 +37,7 @@ struct Shared {
     unsigned long long pc[kPhaseSlots];  // per-phase SM cycles (thread 0, when profiled)
     int opos[kMaxOverrides];
     double2 oval[kMaxOverrides];
+    int orow[kMaxOverrides], ocol[kMaxOverrides];  // the overrides' rows and columns
     int novr;
     int job;
     int piv_err;
@@ -138,71 +140,139 @@ __device__ __forceinline__ double2 ybus_value(const DevPlan &P, const Shared &S,
 }
 
 
-// (Ybus V)[r], over the row's entries in column order
-__device__ __forceinline__ double2 ybus_row_product(const DevPlan &P, const Shared &S, const double2 *__restrict__ V,
-                                                    int r) {
-    double2 s = make_double2(0.0, 0.0);
-    const int p0 = P.Rp[r], p1 = P.Rp[r + 1];
-    for (int p = p0; p < p1; p += 4) {
-        // indices first, then values: the loads of four entries are in flight together
+// Stages override i of an instance (caller: one thread per override).
+__device__ __forceinline__ void stage_override(const DevPlan &P, Shared &S, int i, int pos, double2 val) {
+    S.opos[i] = pos;
+    S.oval[i] = val;
+    S.orow[i] = P.Rrow[pos];
+    S.ocol[i] = P.Rj[pos];
+}
+
+// The overrides that lie in row r, as a bit mask: rows without one (nearly all) then test nothing
+// per entry.
+__device__ __forceinline__ unsigned row_overrides(const Shared &S, int r) {
+    unsigned mask = 0;
+    for (int i = 0; i < S.novr; ++i) mask |= (unsigned)(S.orow[i] == r) << i;
+    return mask;
+}
+
+__device__ __forceinline__ double2 override_value(const Shared &S, unsigned mask, int c, double2 y) {
+    for (; mask; mask &= mask - 1) {
+        const int i = __ffs(mask) - 1;
+        if (S.ocol[i] == c) y = S.oval[i];
+    }
+    return y;
+}
+
+// (Ybus V)[r] of the row in `slot` (bus r, voltage vr, slice sl): the diagonal, then the off-diagonal
+// entries in column order.  KEEP: t = conj(Y V_c) V_r of every entry goes to T / Td, from which the
+// Jacobian fill and the refinement residual take their values (NaN where V_c is zero, see dsbus).
+// The entries of a slice are 32 consecutive values per step (rows sorted by length, so a
+// slice has almost no padding), and the loads of four steps are issued together.
+template <bool KEEP>
+__device__ __forceinline__ double2 ybus_row(const DevPlan &P, const Shared &S, const double2 *__restrict__ V, int slot,
+                                            int r, double2 vr, int2 sl, double2 *__restrict__ T,
+                                            double2 *__restrict__ Td) {
+    const unsigned mask = row_overrides(S, r);
+    double2 yd = P.dg_val[slot];
+    if (mask) yd = override_value(S, mask, r, yd);
+    double2 s = cmul(yd, vr);
+    if (KEEP) Td[slot] = entry_power(s, vr, vr);
+    const int e0 = sl.x + (slot & 31);
+    for (int u0 = 0; u0 < sl.y; u0 += 4) {
         int c[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) c[u] = p + u < p1 ? P.Rj[p + u] : -1;
-        double2 y[4], vv[4];
+        double2 y[4], v[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            y[u] = c[u] >= 0 ? ybus_value(P, S, p + u) : make_double2(0.0, 0.0);
-            vv[u] = c[u] >= 0 ? V[c[u]] : make_double2(0.0, 0.0);
+            const bool in = u0 + u < sl.y;
+            c[u] = in ? P.off_col[e0 + (u0 + u) * 32] : -1;
+            y[u] = in ? P.off_val[e0 + (u0 + u) * 32] : make_double2(0.0, 0.0);
         }
 #pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = c[u] >= 0 ? V[c[u]] : make_double2(0.0, 0.0);
+#pragma unroll
         for (int u = 0; u < 4; ++u) {
-            s.x += y[u].x * vv[u].x - y[u].y * vv[u].y;
-            s.y += y[u].x * vv[u].y + y[u].y * vv[u].x;
+            if (c[u] < 0) continue;
+            if (mask) y[u] = override_value(S, mask, c[u], y[u]);
+            const double2 b = cmul(y[u], v[u]);
+            s.x += b.x;
+            s.y += b.y;
+            if (KEEP) T[e0 + (u0 + u) * 32] = entry_power(b, v[u], vr);
         }
     }
     return s;
 }
 
-// F at V: writes Ibus, the FP64 mismatch per bus and the permuted right-hand side x;
+// F at V: writes the permuted right-hand side x and, for the Jacobian fill and the residual, per
+// row slot Sd = V conj(Ybus V) and (FB) the FP64 mismatch, per entry T / Td (ybus_row);
 // returns ||F||_inf and a non-finite flag to every thread.
-template <typename XT>
-__device__ void mismatch(const DevPlan &P, Shared &S, const double2 *__restrict__ V, double2 *__restrict__ Ibus,
-                         double2 *__restrict__ Fbus, const double2 *__restrict__ Sbus, XT *x, double &norm,
-                         int &bad) {
+// Bound by the latency of its loads: every pass reads a few hundred KB of L2 data per CTA, which
+// 20 to 24 warps cover only when the loads are coalesced and independent.  Rows by slots (against a
+// thread per CSR row with 16-byte loads 58 bytes apart) and T kept for the fill and the
+// residual (against a second and third gather of both voltages per entry) are what that takes.
+template <typename XT, bool FB>
+__device__ void mismatch(const DevPlan &P, Shared &S, const double2 *__restrict__ V, double2 *__restrict__ T,
+                         double2 *__restrict__ Td, double2 *__restrict__ Sd, double2 *__restrict__ Fb,
+                         const double2 *__restrict__ Sbus, XT *x, double &norm, int &bad) {
     double lmax = 0.0;
     int lbad = 0;
     const double sa = S.slack_absorbed;
-    for (int r = threadIdx.x; r < P.n; r += blockDim.x) {
-        // the row's own loads are issued before the row product (they do not depend on it)
-        const double2 sb = __ldcg(Sbus + r);
-        const int ip = P.xP[r], iq = P.xQ[r];
-        const double2 s = ybus_row_product(P, S, V, r);
-        Ibus[r] = s;
-        const double2 vr = V[r];
-        double mr = vr.x * s.x + vr.y * s.y - sb.x;  // V * conj(I) - S
-        const double mi = vr.y * s.x - vr.x * s.y - sb.y;
-        if (P.distributed) mr += sa * P.w[r];
-        Fbus[r] = make_double2(mr, mi);
-        if (ip >= 0) {
-            x[ip] = (XT)mr;
-            lmax = fmax(lmax, fabs(mr));
-            lbad |= !isfinite(mr);
+    const int ns = P.row_slots, bd = blockDim.x;
+    int slot = threadIdx.x;
+    int r = slot < ns ? P.row_bus[slot] : -1;
+    int2 sl = slot < ns ? P.row_slice[slot >> 5] : make_int2(0, 0);
+    while (slot < ns) {
+        // the next slot's row and slice arrive while this one is worked on
+        const int nslot = slot + bd;
+        const int nr = nslot < ns ? P.row_bus[nslot] : -1;
+        const int2 nsl = nslot < ns ? P.row_slice[nslot >> 5] : make_int2(0, 0);
+        if (r >= 0) {
+            const double2 sb = __ldcg(Sbus + r);
+            const int2 eq = P.dg_eq[slot];
+            const double2 vr = V[r];
+            const double2 s = ybus_row<true>(P, S, V, slot, r, vr, sl, T, Td);
+            const double2 d = cmul(cconj(s), vr);  // V * conj(I)
+            Sd[slot] = d;
+            double mr = d.x - sb.x;
+            const double mi = d.y - sb.y;
+            if (P.distributed) mr += sa * P.w[r];
+            if (FB) Fb[slot] = make_double2(mr, mi);
+            if (eq.x >= 0) {
+                x[eq.x] = (XT)mr;
+                lmax = fmax(lmax, fabs(mr));
+                lbad |= !isfinite(mr);
+            }
+            if (eq.y >= 0) {
+                x[eq.y] = (XT)mi;
+                lmax = fmax(lmax, fabs(mi));
+                lbad |= !isfinite(mi);
+            }
         }
-        if (iq >= 0) {
-            x[iq] = (XT)mi;
-            lmax = fmax(lmax, fabs(mi));
-            lbad |= !isfinite(mi);
-        }
+        slot = nslot;
+        r = nr;
+        sl = nsl;
     }
     block_norm(S, lmax, lbad, norm, bad);
 }
 
-// dS/dVm and dS/dVa at V scattered into the LU array (and into Jout when requested).
+// The four Jacobian values of an entry to their LU positions (-1: none).
+template <typename LT>
+__device__ __forceinline__ void put_entry(LT *lu, int4 t, double2 te, double2 d) {
+    double dvar, dvai;
+    double2 dvm;
+    dsbus(te, d, dvar, dvai, dvm);
+    if (t.x >= 0) lu[t.x] = (LT)dvar;
+    if (t.y >= 0) lu[t.y] = (LT)dvai;
+    if (t.z >= 0) lu[t.z] = (LT)dvm.x;
+    if (t.w >= 0) lu[t.w] = (LT)dvm.y;
+}
+
+// dS/dVa and |V| dS/d|V| scattered into the LU array, from the mismatch's T, Td and Sd: every load is coalesced and none depends on another.
 // ZERO_ALL: the LU region (shared memory) is cleared whole with 16-byte stores before the
 // entries are written, in place of the gather of the fill-in positions.
 template <typename LT, bool ZERO_ALL>
-__device__ void jacobian_fill(const DevPlan &P, Shared &S, const double2 *__restrict__ V,
-                              const double2 *__restrict__ Ibus, LT *lu, double *Jout) {
+__device__ void jacobian_fill(const DevPlan &P, const double2 *__restrict__ T, const double2 *__restrict__ Td,
+                              const double2 *__restrict__ Sd, LT *lu) {
     if constexpr (ZERO_ALL) {
         // lu is 4-byte aligned; the head up to the first 16-byte boundary and the tail are scalar
         const int head = (int)(((16 - ((size_t)lu & 15)) & 15) / sizeof(LT));
@@ -215,58 +285,30 @@ __device__ void jacobian_fill(const DevPlan &P, Shared &S, const double2 *__rest
         if ((int)threadIdx.x < P.nnzLU - t0) lu[t0 + threadIdx.x] = (LT)0;
         __syncthreads();
     }
-    constexpr int U = 2;  // entries per thread whose loads are issued together
+    constexpr int U = 4;  // entries per thread whose loads are issued together
     const int bd = blockDim.x;
-    for (int p0 = threadIdx.x; p0 < P.nnzY; p0 += U * bd) {
-        int r[U], c[U];
-        double2 y[U], vr[U], vc[U], ib[U];
+    const double2 zero = make_double2(0.0, 0.0);
+    for (int e0 = threadIdx.x; e0 < P.row_len; e0 += U * bd) {
         int4 t[U];
+        double2 te[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int p = p0 + u * bd;
-            const bool ok = p < P.nnzY;
-            r[u] = ok ? P.Rrow[p] : 0;
-            c[u] = ok ? P.Rj[p] : 1;
-            t[u] = ok ? P.ytarget[p] : make_int4(-1, -1, -1, -1);
+            const int e = e0 + u * bd;
+            const bool ok = e < P.row_len;
+            t[u] = ok ? P.off_target[e] : make_int4(-1, -1, -1, -1);
+            te[u] = ok ? T[e] : zero;  // padding: no target
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int p = p0 + u * bd;
-            const bool ok = p < P.nnzY;
-            y[u] = ok ? ybus_value(P, S, p) : make_double2(0.0, 0.0);
-            vr[u] = ok ? V[r[u]] : make_double2(1.0, 0.0);
-            vc[u] = ok ? V[c[u]] : make_double2(1.0, 0.0);
-            ib[u] = (ok && r[u] == c[u]) ? Ibus[r[u]] : make_double2(0.0, 0.0);
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int p = p0 + u * bd;
-            if (p >= P.nnzY) break;
-            double dvar, dvai;
-            double2 dvm;
-            dsbus(y[u], vr[u], vc[u], r[u] == c[u], ib[u], dvar, dvai, dvm);
-            if (t[u].x >= 0) lu[t[u].x] = (LT)dvar;
-            if (t[u].y >= 0) lu[t[u].y] = (LT)dvai;
-            if (t[u].z >= 0) lu[t[u].z] = (LT)dvm.x;
-            if (t[u].w >= 0) lu[t[u].w] = (LT)dvm.y;
-            if (Jout) {
-                const int4 j = P.yjpos[p];
-                if (j.x >= 0) Jout[j.x] = dvar;
-                if (j.y >= 0) Jout[j.y] = dvai;
-                if (j.z >= 0) Jout[j.z] = dvm.x;
-                if (j.w >= 0) Jout[j.w] = dvm.y;
-            }
-        }
+        for (int u = 0; u < U; ++u) put_entry<LT>(lu, t[u], te[u], zero);
+    }
+    for (int s = threadIdx.x; s < P.row_slots; s += bd) {
+        if (P.dg_pos[s] < 0) continue;
+        put_entry<LT>(lu, P.dg_target[s], Td[s], Sd[s]);
     }
     if constexpr (!ZERO_ALL)
         for (int i = threadIdx.x; i < P.nfill; i += blockDim.x) lu[P.fillpos[i]] = (LT)0;
-    for (int i = threadIdx.x; i < P.nconst; i += blockDim.x) {
-        lu[P.cpos[i]] = (LT)P.cval[i];
-        if (Jout) Jout[P.cjpos[i]] = P.cval[i];
-    }
+    for (int i = threadIdx.x; i < P.nconst; i += blockDim.x) lu[P.cpos[i]] = (LT)P.cval[i];
 }
-
-
 
 template <typename LT, typename XT>
 __device__ __forceinline__ void run_op(const int4 o, LT *lu, XT *v) {
@@ -464,59 +506,69 @@ __device__ void check_pivots(const DevPlan &P, Shared &S, const LT *lu) {
     __syncthreads();
 }
 
-// FP64 residual of the Newton system, F - J dx, written as the next right-hand side.  J is the
-// linearisation of S(V) = V conj(Y V) in the polar unknowns (the dS/dVa, dS/dVm of
-// BaseNRAlgo::_dSbus_dV, BaseNRAlgo.tpp:228-257), so J dx is formed from the voltage
-// step dV = V / |V| dVm + j V dVa:  J dx = dV conj(I) + V conj(Y dV)  (I = Y V, the current
-// injections of the mismatch), plus the slack-absorption column of a distributed slack.
-// Two passes: dV per bus into the slab, then one Ybus row product per equation row.  Returns
-// max |F - J dx| to every thread (infinity when a value is not finite).
+// FP64 residual of the Newton system, F - J dx, into rt (as a right-hand side), for the step x
+// (dVa and u = dVm / |V|, FP32 values taken exactly).  Row r of J dx is the sum over its entries of
+// dS/dVa dVa + |V| dS/d|V| u = t (u - j dVa), plus d (u_r + j dVa_r) of the diagonal (d = V conj(I);
+// the dS/dVa, dS/dVm of BaseNRAlgo::_dSbus_dV, BaseNRAlgo.tpp:228-257), plus the slack-absorption
+// column of a distributed slack: one pass over the mismatch's T, the step gathered from shared
+// memory.  Returns max |F - J dx| to every thread (infinity when a value is not finite).
 template <typename XT>
-__device__ double newton_residual(const DevPlan &P, Shared &S, const double2 *__restrict__ V,
-                                const double2 *__restrict__ Ibus, const double2 *__restrict__ Fbus,
-                                const double *__restrict__ dxg, double2 *__restrict__ dV, XT *x) {
-    const int bd = blockDim.x;
-    for (int b0 = threadIdx.x; b0 < P.n; b0 += 2 * bd) {
-        int ia[2], im[2];
-        double2 v[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int b = b0 + i * bd;
-            const bool ok = b < P.n;
-            ia[i] = ok ? P.xVa[b] : -1;
-            im[i] = ok ? P.xVm[b] : -1;
-            v[i] = ok ? V[b] : make_double2(1.0, 0.0);
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int b = b0 + i * bd;
-            if (b >= P.n) break;
-            const double dA = ia[i] >= 0 ? dxg[ia[i]] : 0.0;
-            const double dM = im[i] >= 0 ? dxg[im[i]] / cabs2(v[i]) : 0.0;
-            dV[b] = make_double2(v[i].x * dM - v[i].y * dA, v[i].y * dM + v[i].x * dA);  // V (dM/|V| + j dA)
-        }
-    }
-    __syncthreads();
+__device__ double newton_residual(const DevPlan &P, Shared &S, const double2 *__restrict__ T,
+                                  const double2 *__restrict__ Td, const double2 *__restrict__ Sd,
+                                  const double2 *__restrict__ Fb, const XT *x, XT *__restrict__ rt) {
+    const int ns = P.row_slots, bd = blockDim.x;
     double lmax = 0.0;
     int lbad = 0;
-    for (int r = threadIdx.x; r < P.n; r += bd) {
-        const int ip = P.xP[r], iq = P.xQ[r];
-        if (ip < 0 && iq < 0) continue;
-        const double2 yd = ybus_row_product(P, S, dV, r);
-        const double2 vr = V[r], dvr = dV[r], ir = Ibus[r];
-        double jP = dvr.x * ir.x + dvr.y * ir.y + (vr.x * yd.x + vr.y * yd.y);
-        const double jQ = dvr.y * ir.x - dvr.x * ir.y + (vr.y * yd.x - vr.x * yd.y);
-        if (P.distributed && ip >= 0) jP += P.wJ[r] * dxg[P.xSlack];
-        const double2 F = Fbus[r];
-        if (ip >= 0) {
-            const double rp = F.x - jP;
-            x[ip] = (XT)rp;
+    for (int slot = threadIdx.x; slot < ns; slot += bd) {
+        const int2 sl = P.row_slice[slot >> 5];
+        const int2 eq = P.dg_eq[slot], ix = P.dg_x[slot];
+        const double2 td = Td[slot], d = Sd[slot], F = Fb[slot];
+        const int e0 = sl.x + (slot & 31);
+        double2 j = make_double2(0.0, 0.0);
+        for (int u0 = 0; u0 < sl.y; u0 += 4) {
+            int2 i[4];
+            double2 t[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool in = u0 + u < sl.y;
+                i[u] = in ? P.off_x[e0 + (u0 + u) * 32] : make_int2(-1, -1);
+                t[u] = in ? T[e0 + (u0 + u) * 32] : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (i[u].x >= 0) {
+                    const double a = (double)x[i[u].x];
+                    j.x += t[u].y * a;
+                    j.y -= t[u].x * a;
+                }
+                if (i[u].y >= 0) {
+                    const double m = (double)x[i[u].y];
+                    j.x += t[u].x * m;
+                    j.y += t[u].y * m;
+                }
+            }
+        }
+        if (eq.x < 0 && eq.y < 0) continue;
+        if (ix.x >= 0) {
+            const double a = (double)x[ix.x];
+            j.x += (td.y - d.y) * a;
+            j.y -= (td.x - d.x) * a;
+        }
+        if (ix.y >= 0) {
+            const double m = (double)x[ix.y];
+            j.x += (td.x + d.x) * m;
+            j.y += (td.y + d.y) * m;
+        }
+        if (P.distributed && eq.x >= 0) j.x += P.wJ[P.row_bus[slot]] * (double)x[P.xSlack];
+        if (eq.x >= 0) {
+            const double rp = F.x - j.x;
+            rt[eq.x] = (XT)rp;
             lmax = fmax(lmax, fabs(rp));
             lbad |= !isfinite(rp);
         }
-        if (iq >= 0) {
-            const double rq = F.y - jQ;
-            x[iq] = (XT)rq;
+        if (eq.y >= 0) {
+            const double rq = F.y - j.y;
+            rt[eq.y] = (XT)rq;
             lmax = fmax(lmax, fabs(rq));
             lbad |= !isfinite(rq);
         }
@@ -526,8 +578,9 @@ __device__ double newton_residual(const DevPlan &P, Shared &S, const double2 *__
     block_norm(S, lmax, lbad, rmax, bad);
     return bad ? INFINITY : rmax;
 }
-// The voltage update of a Newton step: Va -= dVa, Vm -= dVm (the FP32 step x; when refined, the
-// FP64 first step dxg plus xw times the correction x, xw = 0 when the correction was skipped),
+
+// The voltage update of a Newton step: Va -= dVa, Vm -= |V| (dVm / |V|) (the step x; when corrected,
+// the first step dx plus the correction x, added in FP64),
 // V = Vm e^(j Va) into the slab (and the shared copy Vs); returns the thread's smallest new
 // magnitude.  Pairs of buses: their loads (magnitudes and angles, step positions, then
 // the step values) are issued together before the arithmetic of the first bus.
@@ -539,8 +592,7 @@ __device__ double newton_residual(const DevPlan &P, Shared &S, const double2 *__
 template <typename XT>
 __device__ double voltage_update(const DevPlan &P, double2 *__restrict__ V, double2 *__restrict__ Vs,
                                            double *__restrict__ Vm, double *__restrict__ Va,
-                                           const double *__restrict__ dxg, const XT *x, bool refine_now,
-                                           double xw) {
+                                           const XT *__restrict__ dx, const XT *x, bool corrected) {
     const int n = P.n;
     double lmin = 1.0;
     constexpr int R = 2;
@@ -560,8 +612,8 @@ __device__ double voltage_update(const DevPlan &P, double2 *__restrict__ V, doub
         double da[R], dm[R];
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-            da[i] = ia[i] >= 0 ? (refine_now ? dxg[ia[i]] + xw * (double)x[ia[i]] : (double)x[ia[i]]) : 0.0;
-            dm[i] = im[i] >= 0 ? (refine_now ? dxg[im[i]] + xw * (double)x[im[i]] : (double)x[im[i]]) : 0.0;
+            da[i] = ia[i] >= 0 ? (double)x[ia[i]] + (corrected ? (double)dx[ia[i]] : 0.0) : 0.0;
+            dm[i] = im[i] >= 0 ? (double)x[im[i]] + (corrected ? (double)dx[im[i]] : 0.0) : 0.0;
         }
 #pragma unroll
         for (int i = 0; i < R; ++i) {
@@ -569,7 +621,7 @@ __device__ double voltage_update(const DevPlan &P, double2 *__restrict__ V, doub
             if (b >= n) break;
             double a = va[i], mg = vm[i];
             if (ia[i] >= 0) a -= da[i];
-            if (im[i] >= 0) mg -= dm[i];
+            if (im[i] >= 0) mg -= mg * dm[i];  // the unknown is dVm / |V|, and mg = |V|
             double sn, cs;
             sincos(a, &sn, &cs);
             const double2 v = make_double2(mg * cs, mg * sn);
@@ -1011,16 +1063,23 @@ __device__ __noinline__ void tail_backward(const DevPlan &P, Shared &S, const LT
 
 // Where one plan's data lives for a CTA: shared memory x | LU (LU_SMEM: one index space, LU at
 // element lu_offset) | phase tables, and the CTA's slab of the scratch memory.
-// slab bytes per bus: V, Ibus, Fbus, the refinement's voltage step dV (16 B each), Vm, Va (8 B each)
-constexpr size_t kBusSlabBytes = 80;
+// The slab's part before the LU: V (16 B per bus), Vm, Va (8 B per bus), Td, Sd (16 B per row
+// slot), T (16 B per off-diagonal slot); FP32 plans also the FP64 mismatch (16 B per row slot), the
+// first step of a refinement and its residual (a value per unknown).
+__host__ __device__ inline size_t bus_slab_bytes(const DevPlan &P, int x_bytes) {
+    size_t b = (size_t)P.n * 32 + (size_t)P.row_slots * 32 + (size_t)P.row_len * 16;
+    if (x_bytes == 4) b += (size_t)P.row_slots * 16 + (size_t)P.m * 8;
+    return (b + 255) & ~(size_t)255;
+}
 template <typename LT, typename XT>
 struct Layout {
     XT *x;
     LT *lu;
     LT *D;    // dense tail block (global-memory LU plans with a tail)
     LT *tsm;  // its staging area in shared memory
-    double2 *V, *Ibus, *Fbus, *dV;
-    double *Vm, *Va, *dxg;
+    double2 *V, *Td, *Sd, *T, *Fb;
+    double *Vm, *Va;
+    XT *dx, *rt;
     int *sb_fac, *sb_bwd, *sb_fwd, *sw_fac, *sw_bwd, *sw_fwd;
     uint2 *nar_ops[3];  // staged operations of the narrow phases (packed layout)
 };
@@ -1031,15 +1090,20 @@ __device__ __forceinline__ Layout<LT, XT> make_layout(const DevPlan &P, const Ba
     const int n = P.n, m = P.m;
     const size_t xbytes = LU_SMEM ? (size_t)P.lu_offset * sizeof(XT) : (((size_t)m * sizeof(XT) + 15) & ~(size_t)15);
     L.x = reinterpret_cast<XT *>(dyn);
+    // opaque to the optimiser: every pass of a Newton step derives its pointers again instead of
+    // keeping all of them live (or spilled) across the others
     unsigned char *slab = A.scratch + (size_t)blockIdx.x * (size_t)A.slab_bytes;
+    asm volatile("" : "+l"(slab));
     L.V = reinterpret_cast<double2 *>(slab);
-    L.Ibus = L.V + n;
-    L.Fbus = L.Ibus + n;
-    L.dV = L.Fbus + n;
-    L.Vm = reinterpret_cast<double *>(L.dV + n);
+    L.Td = L.V + n;
+    L.Sd = L.Td + P.row_slots;
+    L.T = L.Sd + P.row_slots;
+    L.Vm = reinterpret_cast<double *>(L.T + P.row_len);
     L.Va = L.Vm + n;
-    L.dxg = L.Va + n;
-    const size_t bus_bytes = (((size_t)n * kBusSlabBytes + (size_t)m * 8) + 255) & ~(size_t)255;
+    L.Fb = reinterpret_cast<double2 *>(L.Va + n);  // FP32 plans: Fb, dx, rt
+    L.dx = reinterpret_cast<XT *>(L.Fb + P.row_slots);
+    L.rt = L.dx + m;
+    const size_t bus_bytes = bus_slab_bytes(P, sizeof(XT));
     L.lu = LU_SMEM ? reinterpret_cast<LT *>(dyn + xbytes) : reinterpret_cast<LT *>(slab + bus_bytes);
     L.D = LU_SMEM ? nullptr
                   : reinterpret_cast<LT *>(slab + bus_bytes + (((size_t)P.nnzLU * sizeof(LT) + 255) & ~(size_t)255));
@@ -1109,42 +1173,44 @@ struct Prof {
 // NARROW: the narrow phases of the packed programs run on their few warps (the 512- and
 // 640-thread variants; at 768 threads the registers it takes cost more than it saves).
 template <typename LT, typename XT, bool LU_SMEM, bool REFINE, bool NARROW>
-__device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, Shared &S, const Layout<LT, XT> &L,
-                                          int first, int count, Prof &pr) {
+__device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, Shared &S, unsigned char *dyn, int first, int count, Prof &pr) {
     const int tid = threadIdx.x;
     const int n = P.n, m = P.m;
-    XT *x = L.x;
-    LT *lu = L.lu;
-    double2 *V = L.V, *Ibus = L.Ibus, *Fbus = L.Fbus;
-    double *Vm = L.Vm, *Va = L.Va, *dxg = L.dxg;
+    const auto lay = [&]() { return make_layout<LT, XT, LU_SMEM>(P, A, dyn); };
+    XT *const x = reinterpret_cast<XT *>(dyn);
     // With the LU in shared memory, the LU region is dead from the voltage update to the next
     // Jacobian fill: the voltages are also written there (Vs) and the mismatch gathers them from
     // shared memory instead of the slab.  Not when the LU must survive the mismatch (LU reuse).
     double2 *Vs = nullptr;
     if constexpr (LU_SMEM) {
         if (!(REFINE && A.reuse_below > 0.0) && (size_t)n * sizeof(double2) <= (size_t)P.nnzLU * sizeof(LT))
-            Vs = reinterpret_cast<double2 *>(lu);
+            Vs = reinterpret_cast<double2 *>(lay().lu);
     }
     for (int step = 0; step < count; ++step) {
         const int inst = first + step;
         const double2 *Sb = A.Sbus + (long long)inst * A.sbus_stride;
         if (step == 0 || !A.chain) {
+            const Layout<LT, XT> L = lay();
             const double2 *v0 = A.v0_from_out ? out_row(A, inst, n) : A.V0 + (long long)inst * A.v0_stride;
             for (int b = tid; b < n; b += blockDim.x) {
                 const double2 v = __ldcg(v0 + b);
-                V[b] = v;
+                L.V[b] = v;
                 if (Vs) Vs[b] = v;
-                Vm[b] = cabs2(v);
-                Va[b] = atan2(v.y, v.x);
+                L.Vm[b] = cabs2(v);
+                L.Va[b] = atan2(v.y, v.x);
             }
         } else {
+            const Layout<LT, XT> L = lay();
             for (int b = tid; b < n; b += blockDim.x) {
-                const double2 v = V[b];
+                const double2 v = L.V[b];
                 if (Vs) Vs[b] = v;
-                Vm[b] = cabs2(v);
-                Va[b] = atan2(v.y, v.x);
+                L.Vm[b] = cabs2(v);
+                L.Va[b] = atan2(v.y, v.x);
             }
         }
+        // the mismatch reads the injections in row-slot order: bring the row into L2 in bus order first
+        for (int b = 8 * tid; b < n; b += 8 * blockDim.x)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(Sb + b));
         if (tid == 0) {
             int k0 = 0, k1 = 0;
             if (A.ovr_ptr) {
@@ -1158,8 +1224,7 @@ __device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, 
         __syncthreads();
         if (tid < S.novr) {
             const int k0 = __ldcg(A.ovr_ptr + inst);
-            S.opos[tid] = __ldcg(A.ovr_pos + k0 + tid);
-            S.oval[tid] = __ldcg(A.ovr_val + k0 + tid);
+            stage_override(P, S, tid, __ldcg(A.ovr_pos + k0 + tid), __ldcg(A.ovr_val + k0 + tid));
         }
         if (P.distributed) {
             double ls = 0.0;
@@ -1171,6 +1236,7 @@ __device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, 
         if (S.novr < 0) {
             // more Ybus overrides than the kernel stages: not computed (start voltages out)
             double2 *vo = out_row(A, inst, n);
+            const double2 *V = lay().V;
             for (int b = tid; b < n; b += blockDim.x) vo[b] = A.zero_failed ? make_double2(0.0, 0.0) : V[b];
             if (tid == 0) {
                 A.iters[inst] = 0;
@@ -1188,14 +1254,33 @@ __device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, 
         }
         double norm;
         int bad;
+        const auto step_mismatch = [&]() {
+            const Layout<LT, XT> L = lay();
+            mismatch<XT, REFINE>(P, S, Vs ? Vs : L.V, L.T, L.Td, L.Sd, L.Fb, Sb, x, norm, bad);
+        };
         pr.mark(6);
-        mismatch<XT>(P, S, Vs ? Vs : V, Ibus, Fbus, Sb, x, norm, bad);
+        step_mismatch();
         pr.mark(0);
         bool conv = !bad && norm < A.tol;
         int it = A.it_start ? A.it_start[inst] : 0, err = 0;
-        double *Jout = (A.Jout && inst == A.j_inst) ? A.Jout : nullptr;
+        double2 *const Vlast = inst == A.j_inst ? A.Vlast : nullptr;
         Trace tr{(A.trace != nullptr && blockIdx.x == 0 && pr.traced == 0) ? A.trace : nullptr, A.trace_cap, 0};
         pr.traced = 1;
+        const auto program_factor = [&]() {
+            const Layout<LT, XT> L = lay();
+            run_lu_program<LT, XT, LU_SMEM, NARROW>(P.fac_cops, P.fac_ops, L.sb_fac, L.sw_fac, P.fac_nph, m, L.lu, x,
+                                                    tr, make_int3(P.nar_a[0], P.nar_b[0], P.nar_warps), L.nar_ops[0]);
+        };
+        const auto program_backward = [&]() {
+            const Layout<LT, XT> L = lay();
+            run_lu_program<LT, XT, LU_SMEM, NARROW>(P.bwd_cops, P.bwd_ops, L.sb_bwd, L.sw_bwd, P.bwd_nph, m, L.lu, x,
+                                                    tr, make_int3(P.nar_a[1], P.nar_b[1], P.nar_warps), L.nar_ops[1]);
+        };
+        const auto program_forward = [&]() {
+            const Layout<LT, XT> L = lay();
+            run_lu_program<LT, XT, LU_SMEM, NARROW>(P.fwd_cops, P.fwd_ops, L.sb_fwd, L.sw_fwd, P.fwd_nph, m, L.lu, x,
+                                                    tr, make_int3(P.nar_a[2], P.nar_b[2], P.nar_warps), L.nar_ops[2]);
+        };
         bool have_lu = false;  // this instance's LU from an earlier iteration is in place
         while (!conv && it < A.max_iter) {
             ++it;
@@ -1203,39 +1288,41 @@ __device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, 
             // close to the solution the Jacobian barely moves between iterations: the step is
             // solved with the previous iteration's LU and refined against the current FP64
             // Jacobian (refine_now holds: reuse_below <= refine_below)
-            const bool reuse = REFINE && have_lu && Jout == nullptr && norm < A.reuse_below;
+            const bool reuse = REFINE && have_lu && Vlast == nullptr && norm < A.reuse_below;
             tr.mark();
+            if (Vlast)  // one instance of a single power flow
+                for (int b = tid; b < n; b += blockDim.x) Vlast[b] = lay().V[b];
             if (!reuse) {
-                jacobian_fill<LT, LU_SMEM>(P, S, V, Ibus, lu, Jout);
+                {
+                    const Layout<LT, XT> L = lay();
+                    jacobian_fill<LT, LU_SMEM>(P, L.T, L.Td, L.Sd, L.lu);
+                }
                 __syncthreads();
                 pr.mark(1);
                 // refactorisation with the forward substitution of the right-hand side fused in
-                run_lu_program<LT, XT, LU_SMEM, NARROW>(P.fac_cops, P.fac_ops, L.sb_fac, L.sw_fac, P.fac_nph, m, lu, x, tr,
-                                                make_int3(P.nar_a[0], P.nar_b[0], P.nar_warps), L.nar_ops[0]);
+                program_factor();
                 if constexpr (!LU_SMEM) {
                     if (P.tail_k > 0) {
-                        tail_factor<LT>(P, lu, L.D, L.tsm);
-                        tail_forward<LT, XT>(P, L.D, x, L.tsm);
+                        tail_factor<LT>(P, lay().lu, lay().D, lay().tsm);
+                        tail_forward<LT, XT>(P, lay().D, x, lay().tsm);
                     }
                 }
                 pr.mark(2);
                 have_lu = true;
             } else {
-                run_lu_program<LT, XT, LU_SMEM, NARROW>(P.fwd_cops, P.fwd_ops, L.sb_fwd, L.sw_fwd, P.fwd_nph, m, lu, x, tr,
-                                                make_int3(P.nar_a[2], P.nar_b[2], P.nar_warps), L.nar_ops[2]);
+                program_forward();
                 if constexpr (!LU_SMEM) {
-                    if (P.tail_k > 0) tail_forward<LT, XT>(P, L.D, x, L.tsm);
+                    if (P.tail_k > 0) tail_forward<LT, XT>(P, lay().D, x, lay().tsm);
                 }
                 pr.mark(3);
             }
             if constexpr (!LU_SMEM) {
-                if (P.tail_k > 0) tail_backward<LT, XT>(P, S, L.D, x, L.tsm);
+                if (P.tail_k > 0) tail_backward<LT, XT>(P, S, lay().D, x, lay().tsm);
             }
-            run_lu_program<LT, XT, LU_SMEM, NARROW>(P.bwd_cops, P.bwd_ops, L.sb_bwd, L.sw_bwd, P.bwd_nph, m, lu, x, tr,
-                                            make_int3(P.nar_a[1], P.nar_b[1], P.nar_warps), L.nar_ops[1]);
+            program_backward();
             // a zero pivot of the refactorisation is detected here: the backward program ran on
             // non-finite values, which are dropped with the step
-            scale_by_pivots<LT, XT, true>(P, S, lu, x);
+            scale_by_pivots<LT, XT, true>(P, S, lay().lu, x);
             if (S.piv_err) {
                 err = 6;  // SolverReFactor
                 break;
@@ -1244,40 +1331,43 @@ __device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, 
             // the refinement's correction solve is skipped when the residual of the FP32 step is
             // below a hundredth of the tolerance: the correction would move the next mismatch by
             // less than that (J e = r), and the final voltages by at most |J^-1| tol / 100
-            double xw = 1.0;
-            if (refine_now) {
-                for (int k = tid; k < m; k += blockDim.x) dxg[k] = (double)x[k];
-                __syncthreads();
-                const double rmax = newton_residual<XT>(P, S, V, Ibus, Fbus, dxg, L.dV, x);
-                if (rmax < 0.01 * A.tol) xw = 0.0;
+            bool corrected = false;
+            if constexpr (REFINE) {
+                if (refine_now) {
+                    const Layout<LT, XT> L = lay();
+                    corrected = !(newton_residual<XT>(P, S, L.T, L.Td, L.Sd, L.Fb, x, L.rt) < 0.01 * A.tol);
+                }
             }
-            if (refine_now && xw != 0.0) {
+            if (corrected) {
+                const Layout<LT, XT> L = lay();
+                for (int k = tid; k < m; k += blockDim.x) {
+                    L.dx[k] = x[k];
+                    x[k] = L.rt[k];
+                }
                 __syncthreads();
-                run_lu_program<LT, XT, LU_SMEM, NARROW>(P.fwd_cops, P.fwd_ops, L.sb_fwd, L.sw_fwd, P.fwd_nph, m, lu, x, tr,
-                                                make_int3(P.nar_a[2], P.nar_b[2], P.nar_warps), L.nar_ops[2]);
+                program_forward();
                 if constexpr (!LU_SMEM) {
                     if (P.tail_k > 0) {
-                        tail_forward<LT, XT>(P, L.D, x, L.tsm);
-                        tail_backward<LT, XT>(P, S, L.D, x, L.tsm);
+                        tail_forward<LT, XT>(P, lay().D, x, lay().tsm);
+                        tail_backward<LT, XT>(P, S, lay().D, x, lay().tsm);
                     }
                 }
-                run_lu_program<LT, XT, LU_SMEM, NARROW>(P.bwd_cops, P.bwd_ops, L.sb_bwd, L.sw_bwd, P.bwd_nph, m, lu, x, tr,
-                                            make_int3(P.nar_a[1], P.nar_b[1], P.nar_warps), L.nar_ops[1]);
-                scale_by_pivots<LT, XT>(P, S, lu, x);
+                program_backward();
+                scale_by_pivots<LT, XT>(P, S, lay().lu, x);
             }
             if (refine_now) pr.mark(5);
             // voltage update
-            const double lmin = voltage_update<XT>(P, V, Vs, Vm, Va, dxg, x, refine_now, xw);
+            const Layout<LT, XT> L = lay();
+            const double lmin = voltage_update<XT>(P, L.V, Vs, L.Vm, L.Va, L.dx, x, corrected);
             if (P.distributed) {
-                const double dxs =
-                    refine_now ? dxg[P.xSlack] + xw * (double)x[P.xSlack] : (double)x[P.xSlack];
+                const double dxs = (double)x[P.xSlack] + (corrected ? (double)L.dx[P.xSlack] : 0.0);
                 const double vmin = block_min(S, lmin);  // contains barriers
                 if (tid == 0) S.slack_absorbed -= dxs;
                 if (vmin < 0.0) {
                     for (int b = tid; b < n; b += blockDim.x) {
-                        const double2 v = V[b];
-                        Vm[b] = cabs2(v);
-                        Va[b] = atan2(v.y, v.x);
+                        const double2 v = L.V[b];
+                        L.Vm[b] = cabs2(v);
+                        L.Va[b] = atan2(v.y, v.x);
                     }
                 }
             }
@@ -1285,7 +1375,7 @@ __device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, 
             tr.mark();
             tr.buf = nullptr;
             pr.mark(6);
-            mismatch<XT>(P, S, Vs ? Vs : V, Ibus, Fbus, Sb, x, norm, bad);
+            step_mismatch();
             pr.mark(0);
             if (bad) {
                 err = 3;  // InifiniteValue
@@ -1296,7 +1386,8 @@ __device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, 
         if (!conv && err == 0) err = 2;  // TooManyIterations
         double2 *vo = out_row(A, inst, n);
         const bool zero = A.zero_failed && err != 0;
-        for (int b = tid; b < n; b += blockDim.x) vo[b] = zero ? make_double2(0.0, 0.0) : V[b];
+        const double2 *V = lay().V;
+        for (int b = tid; b < n; b += blockDim.x) __stcs(vo + b, zero ? make_double2(0.0, 0.0) : V[b]);
         if (tid == 0) {
             A.iters[inst] = it;
             A.errs[inst] = err;
@@ -1326,7 +1417,7 @@ __device__ __noinline__ void fp64_rerun(const DevPlan &P, const BatchArgs &A, Sh
     __syncthreads();
     Prof pr;
     pr.start(false, S.pc);
-    solve_job<double, double, false, false, false>(P, A, S, L, first, count, pr);
+    solve_job<double, double, false, false, false>(P, A, S, dyn, first, count, pr);
 }
 
 // QUEUE: the device-resident request loop (jobs from M.q); a variant of its own so that the
@@ -1351,7 +1442,6 @@ __global__ void __launch_bounds__(MAXT, 1) nr_batch_kernel(const DevPlan P0, con
     Prof pr;
     pr.start(A0.phase_cycles != nullptr && tid == 0, S.pc);
     int cur = -1;
-    Layout<LT, XT> L{};
     __shared__ QueueJob qjob;
     for (;;) {
         if constexpr (QUEUE) {
@@ -1386,13 +1476,12 @@ __global__ void __launch_bounds__(MAXT, 1) nr_batch_kernel(const DevPlan P0, con
             }
             __syncthreads();
             cur = sj;
-            L = make_layout<LT, XT, LU_SMEM>(seg.P, seg.A, dyn);
-            stage_tables<LT, XT>(seg.P, L);
+            stage_tables<LT, XT>(seg.P, make_layout<LT, XT, LU_SMEM>(seg.P, seg.A, dyn));
             __syncthreads();
         }
         const int first = queue ? qjob.first : (multi ? M.job_first[job] : A0.job_first[job]);
         const int count = queue ? qjob.count : (multi ? M.job_count[job] : A0.job_count[job]);
-        solve_job<LT, XT, LU_SMEM, REFINE, (MAXT <= 640)>(seg.P, seg.A, S, L, first, count, pr);
+        solve_job<LT, XT, LU_SMEM, REFINE, (MAXT <= 640)>(seg.P, seg.A, S, dyn, first, count, pr);
         __syncthreads();
         if constexpr (REFINE) {
             if (seg.A.fp64_inline) {
@@ -1419,7 +1508,8 @@ __global__ void __launch_bounds__(MAXT, 1) nr_batch_kernel(const DevPlan P0, con
                         seg.A.it_start = its;
                         seg.A.v0_from_out = vfo;
                     }
-                    stage_tables<LT, XT>(seg.P, L);  // the FP64 solve vector covered them
+                    // the FP64 solve vector covered them
+                    stage_tables<LT, XT>(seg.P, make_layout<LT, XT, LU_SMEM>(seg.P, seg.A, dyn));
                     __syncthreads();
                 }
             }
@@ -1496,8 +1586,7 @@ __global__ void __launch_bounds__(512, 1) dc_batch_kernel(const DevPlan P, const
             __syncthreads();
             if (tid < S.novr) {
                 const int k0 = A.ovr_ptr[inst];
-                S.opos[tid] = A.ovr_pos[k0 + tid];
-                S.oval[tid] = A.ovr_val[k0 + tid];
+                stage_override(P, S, tid, A.ovr_pos[k0 + tid], A.ovr_val[k0 + tid]);
             }
             __syncthreads();
             if (S.novr < 0) {
@@ -1649,10 +1738,11 @@ __device__ void fdpf_mismatch(const DevPlan &P, Shared &S, const double2 *__rest
     double lmax = 0.0;
     int lbad = 0;
     const double sa = S.slack_absorbed;
-    for (int r = threadIdx.x; r < P.n; r += blockDim.x) {
-        const double2 s = ybus_row_product(P, S, V, r);
-        const double2 vr = V[r];
-        const double2 sb = Sbus[r];
+    for (int slot = threadIdx.x; slot < P.row_slots; slot += blockDim.x) {
+        const int r = P.row_bus[slot];
+        if (r < 0) continue;
+        const double2 vr = V[r], sb = Sbus[r];
+        const double2 s = ybus_row<false>(P, S, V, slot, r, vr, P.row_slice[slot >> 5], nullptr, nullptr);
         double mr = vr.x * s.x + vr.y * s.y - sb.x;  // V * conj(I) - S + slack_absorbed * w
         double mi = vr.y * s.x - vr.x * s.y - sb.y;
         mr += sa * P.w[r];
@@ -1660,7 +1750,7 @@ __device__ void fdpf_mismatch(const DevPlan &P, Shared &S, const double2 *__rest
         mr /= vm;
         mi /= vm;
         lbad |= !isfinite(mr) || !isfinite(mi);
-        const int ip = P.xP[r], iq = P.xQ[r];
+        const int ip = P.dg_eq[slot].x, iq = P.dg_eq[slot].y;
         if (ip >= 0) {
             if (which == 0) x[ip] = mr;
             lmax = fmax(lmax, fabs(mr));
@@ -1738,8 +1828,7 @@ __global__ void __launch_bounds__(MAXT, MINB) fdpf_batch_kernel(const DevPlan P0
             __syncthreads();
             if (tid < S.novr) {
                 const int k0 = A.ovr_ptr[inst];
-                S.opos[tid] = A.ovr_pos[k0 + tid];
-                S.oval[tid] = A.ovr_val[k0 + tid];
+                stage_override(P, S, tid, A.ovr_pos[k0 + tid], A.ovr_val[k0 + tid]);
             }
             double ls = 0.0;
             for (int b = tid; b < n; b += blockDim.x) ls += Sb[b].x;
@@ -1878,6 +1967,62 @@ int occupancy_variant(int threads, size_t smem) {
     return nb;
 }
 
+// The reference's Jacobian (dS/dVa, dS/d|V|) at V, in J order: a thread per row slot, its row product
+// for the diagonal, then the entries.  A kernel of its own over the whole GPU: written by
+// the one CTA of a single power flow in every iteration it took 20k cycles a time.
+__global__ void jacobian_values_kernel(const DevPlan P, const double2 *__restrict__ V, double *__restrict__ Jout) {
+    for (int slot = blockIdx.x * blockDim.x + threadIdx.x; slot < P.row_slots; slot += gridDim.x * blockDim.x) {
+        const int r = P.row_bus[slot];
+        if (r < 0) continue;
+        const int2 sl = P.row_slice[slot >> 5];
+        const int e0 = sl.x + (slot & 31);
+        const double2 vr = V[r];
+        double2 s = cmul(P.dg_val[slot], vr);
+        const double2 td = cmul(cconj(s), vr);
+        for (int u = 0; u <= sl.y; ++u) {
+            // the off-diagonal entries, then the diagonal (whose value needs the row's sum)
+            const bool diag = u == sl.y;
+            const int e = e0 + 32 * u, p = diag ? P.dg_pos[slot] : P.off_pos[e], c = diag ? r : P.off_col[e];
+            if (p < 0) continue;
+            const double2 vc = V[c];
+            double2 t = td, d = make_double2(0.0, 0.0);
+            if (diag) {
+                d = cmul(cconj(s), vr);
+            } else {
+                const double2 b = cmul(P.off_val[e], vc);
+                s.x += b.x;
+                s.y += b.y;
+                t = cmul(cconj(b), vr);
+            }
+            double dvar, dvai;
+            double2 dvm;
+            dsbus(t, d, dvar, dvai, dvm);
+            const double vm = cabs2(vc);
+            const int4 j = P.yjpos[p];
+            if (j.x >= 0) Jout[j.x] = dvar;
+            if (j.y >= 0) Jout[j.y] = dvai;
+            if (j.z >= 0) Jout[j.z] = dvm.x / vm;
+            if (j.w >= 0) Jout[j.w] = dvm.y / vm;
+        }
+    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.nconst; i += gridDim.x * blockDim.x)
+        Jout[P.cjpos[i]] = P.cval[i];
+}
+
+// Ybus values (storage order) into Rx and the row slots.
+__global__ void set_ybus_kernel(const double2 *__restrict__ src, const int *__restrict__ of_csr, int nnz,
+                                double2 *__restrict__ Rx, double2 *__restrict__ off, double2 *__restrict__ dg) {
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += gridDim.x * blockDim.x) {
+        const double2 y = src[p];
+        if (Rx != src) Rx[p] = y;
+        if (of_csr != nullptr) {
+            const int at = of_csr[p];
+            if (at >= 0) off[at] = y;
+            else dg[-1 - at] = y;
+        }
+    }
+}
+
 // Result rows in case order: row c = the converged voltages of compact instance map[c], or
 // zeros (islanded case, map[c] < 0, or an instance that did not converge).
 __global__ void scatter_case_rows(const double2 *__restrict__ src, const int *__restrict__ errs,
@@ -1900,8 +2045,22 @@ cudaError_t launch_scatter_case_rows(const double2 *src, const int *errs, const 
     return cudaGetLastError();
 }
 
+cudaError_t launch_jacobian_values(const DevPlan &P, const double2 *V, double *Jout, int num_sms, cudaStream_t st) {
+    if (P.row_slots <= 0) return cudaSuccess;
+    jacobian_values_kernel<<<std::min((P.row_slots + 63) / 64, num_sms * 8), 64, 0, st>>>(P, V, Jout);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_set_ybus(const DevPlan &P, const double2 *src, int num_sms, cudaStream_t st) {
+    if (P.nnzY <= 0) return cudaSuccess;
+    set_ybus_kernel<<<std::min((P.nnzY + 255) / 256, num_sms * 8), 256, 0, st>>>(
+        src, P.row_slots > 0 ? P.row_of_csr : nullptr, P.nnzY, const_cast<double2 *>(P.Rx),
+        const_cast<double2 *>(P.off_val), const_cast<double2 *>(P.dg_val));
+    return cudaGetLastError();
+}
+
 size_t slab_bytes(const DevPlan &P, int lu_bytes, bool lu_in_smem) {
-    size_t bus = (((size_t)P.n * kBusSlabBytes + (size_t)P.m * 8) + 255) & ~(size_t)255;
+    size_t bus = bus_slab_bytes(P, lu_bytes);
     size_t lu = lu_in_smem ? 0 : (((size_t)P.nnzLU * lu_bytes + 255) & ~(size_t)255);
     // the dense tail block after the LU (global-memory LU plans only)
     size_t tail = lu_in_smem ? 0 : (((size_t)P.tail_k * (size_t)tail_ld(P.tail_k) * lu_bytes + 255) & ~(size_t)255);

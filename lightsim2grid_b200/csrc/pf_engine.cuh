@@ -16,6 +16,22 @@ struct DevPlan {
     const double *w;
     const int4 *ytarget;   // 4 LU positions per CSR position
     const int4 *yjpos;     // 4 J positions per CSR position
+    // Ybus rows as the one-CTA kernels walk them: slot s is bus row_bus[s] (-1: padding), rows in
+    // decreasing number of off-diagonal entries, a warp per slice of 32 slots; the diagonal per slot
+    // (dg_*), the off-diagonal entries of slice g at [row_slice[g].x + 32 u + lane], u <
+    // row_slice[g].y, in column order (column -1: padding).  row_len: off-diagonal slots.
+    int row_slots, row_len;
+    const int *row_bus;
+    const int2 *row_slice;
+    const int *off_col, *off_pos;  // column, CSR position
+    const double2 *off_val;
+    const int4 *off_target;        // LU positions, as ytarget
+    const int2 *off_x;             // xVa, xVm of the column
+    const int *dg_pos;
+    const double2 *dg_val;
+    const int4 *dg_target;
+    const int2 *dg_eq, *dg_x;      // xP, xQ and xVa, xVm of the slot's bus
+    const int *row_of_csr;         // per CSR position: off-diagonal slot, or -1 - diagonal slot
     const int *fillpos;
     int nfill;
     const int *cpos, *cjpos;
@@ -74,7 +90,7 @@ struct BatchArgs {
     double2 *Vout;            // n per instance
     int *iters;
     int *errs;
-    double *Jout;             // J values (CSC order) of the last iteration of instance j_inst
+    double2 *Vlast;           // optional: the voltages that instance j_inst's last Newton step started from
     int j_inst;
     unsigned char *scratch;   // per-CTA slab
     long long slab_bytes;
@@ -161,6 +177,10 @@ size_t smem_bytes(const DevPlan &P, int lu_bytes, int x_bytes, bool lu_in_smem);
 // A.lu_in_smem and A.refine select the kernel variant.
 cudaError_t launch_nr_batch(const DevPlan &P, const BatchArgs &A, int precision, int threads, int grid,
                             size_t smem, cudaStream_t stream, const MultiArgs &M = MultiArgs{});
+// Ybus values in storage order (device) into the plan's arrays (Rx and the row slots).
+cudaError_t launch_set_ybus(const DevPlan &P, const double2 *src, int num_sms, cudaStream_t st);
+// J values (the reference's, CSC order) of a Newton plan at V (device).
+cudaError_t launch_jacobian_values(const DevPlan &P, const double2 *V, double *Jout, int num_sms, cudaStream_t st);
 // Copies the converged result rows of a compacted batch into case order (zero rows for
 // cases with map[c] < 0 or errs[map[c]] != 0).
 cudaError_t launch_scatter_case_rows(const double2 *src, const int *errs, const int *map, int ncases, int n,

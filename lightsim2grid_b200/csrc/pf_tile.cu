@@ -345,14 +345,15 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
         __syncthreads();
         if (S.nstep > 0) {
             const bool step = S.state[lane] == kStep;
-            // ---- Jacobian values (dS/dVa, dS/dVm) into the LU array
+            // ---- Jacobian values (dS/dVa, |V| dS/d|V|) into the LU array
             if (step) {
                 for (int p = warp; p < P.nnzY; p += kW) {
                     const int r = P.Rrow[p], c = P.Rj[p];
                     double dvar, dvai;
                     double2 dvm;
-                    dsbus(ybus_lane(P, S, p, lane), V[ix(r, lane)], V[ix(c, lane)], r == c,
-                          r == c ? Ib[ix(r, lane)] : make_double2(0.0, 0.0), dvar, dvai, dvm);
+                    const double2 vr = V[ix(r, lane)], vc = V[ix(c, lane)];
+                    dsbus(entry_power(cmul(ybus_lane(P, S, p, lane), vc), vc, vr),
+                          r == c ? cmul(cconj(Ib[ix(r, lane)]), vr) : make_double2(0.0, 0.0), dvar, dvai, dvm);
                     const int4 t = P.ytarget[p];
                     if (t.x >= 0) lu[ix(t.x, lane)] = (LT)dvar;
                     if (t.y >= 0) lu[ix(t.y, lane)] = (LT)dvai;
@@ -397,14 +398,14 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
                 if (refine)
                     for (int k = warp; k < m; k += kW) dxg[ix(k, lane)] = (double)x[ix(k, lane)];
                 __syncthreads();
-                // J dx = dV conj(I) + V conj(Y dV), dV = V / |V| dVm + j V dVa: the linearisation
+                // J dx = dV conj(I) + V conj(Y dV), dV = V (dVm / |V|) + j V dVa: the linearisation
                 // of S(V) = V conj(Y V) that the Jacobian holds (as the one-CTA kernel forms it)
                 if (refine)
                     for (int b = warp; b < n; b += kW) {
                         const int ia = P.xVa[b], im = P.xVm[b];
                         const double2 v = V[ix(b, lane)];
                         const double dA = ia >= 0 ? dxg[ix(ia, lane)] : 0.0;
-                        const double dM = im >= 0 ? dxg[ix(im, lane)] / cabs2(v) : 0.0;
+                        const double dM = im >= 0 ? dxg[ix(im, lane)] : 0.0;  // dVm / |V|
                         dV[ix(b, lane)] = make_double2(v.x * dM - v.y * dA, v.y * dM + v.x * dA);
                     }
                 __syncthreads();
@@ -447,7 +448,8 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
                     double vm = Vm[ix(r, lane)], va = Va[ix(r, lane)];
                     const int ia = P.xVa[r], im = P.xVm[r];
                     if (ia >= 0) va -= refine ? dxg[ix(ia, lane)] + (double)x[ix(ia, lane)] : (double)x[ix(ia, lane)];
-                    if (im >= 0) vm -= refine ? dxg[ix(im, lane)] + (double)x[ix(im, lane)] : (double)x[ix(im, lane)];
+                    if (im >= 0)  // the unknown is dVm / |V|, and vm = |V|
+                        vm -= vm * (refine ? dxg[ix(im, lane)] + (double)x[ix(im, lane)] : (double)x[ix(im, lane)]);
                     double sn, cs;
                     sincos(va, &sn, &cs);
                     const double2 v = make_double2(vm * cs, vm * sn);
