@@ -32,6 +32,8 @@ enum : int { kFree = 0, kNew = 1, kStep = 2, kDone = 3, kIdle = 4 };
 struct TileLanes {
     int inst[kLanes], next[kLanes], end[kLanes], it[kLanes], err[kLanes], state[kLanes], refine[kLanes];
     int novr[kLanes];
+    // the rows of the lane's overrides when they lie in at most two (a branch outage), else row_a -2
+    int row_a[kLanes], row_b[kLanes];
     double sa[kLanes];
     int opos[kMaxOverrides][kLanes];
     double2 oval[kMaxOverrides][kLanes];
@@ -60,11 +62,16 @@ __device__ __forceinline__ unsigned ix(int i, int lane) { return ((unsigned)i <<
 
 __host__ __device__ __forceinline__ size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-__device__ __forceinline__ double2 ybus_lane(const DevPlan &P, const TileLanes &S, int p, int lane) {
+// Ybus entry p of row r for a lane whose overrides lie in rows ra and rb (see TileLanes): the
+// overrides are looked through only there.
+__device__ __forceinline__ double2 ybus_lane(const DevPlan &P, const TileLanes &S, int p, int r, int lane, int ra,
+                                             int rb) {
     double2 y = P.Rx[p];
-    const int no = S.novr[lane];
-    for (int i = 0; i < no; ++i)
-        if (S.opos[i][lane] == p) y = S.oval[i][lane];
+    if (r == ra || r == rb || ra == -2) {
+        const int no = S.novr[lane];
+        for (int i = 0; i < no; ++i)
+            if (S.opos[i][lane] == p) y = S.oval[i][lane];
+    }
     return y;
 }
 
@@ -157,6 +164,7 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
         S.next[tid] = S.end[tid] = 0;
         S.inst[tid] = 0;
         S.novr[tid] = 0;
+        S.row_a[tid] = S.row_b[tid] = -1;
         S.refine[tid] = 0;
     }
     __syncthreads();
@@ -191,13 +199,21 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
                     }
                     if (k1 - k0 > kMaxOverrides) {
                         S.novr[lane] = 0;
+                        S.row_a[lane] = S.row_b[lane] = -1;
                         S.err[lane] = 8;  // NotInitError: more overrides than staged, not computed
                     } else {
                         S.novr[lane] = k1 - k0;
+                        int ra = -1, rb = -1;
                         for (int i = 0; i < k1 - k0; ++i) {
-                            S.opos[i][lane] = A.ovr_pos[k0 + i];
+                            const int pos = A.ovr_pos[k0 + i], r = P.Rrow[pos];
+                            S.opos[i][lane] = pos;
                             S.oval[i][lane] = A.ovr_val[k0 + i];
+                            if (ra == -1 || r == ra) ra = r;
+                            else if (rb == -1 || r == rb) rb = r;
+                            else ra = -2;
                         }
+                        S.row_a[lane] = ra;
+                        S.row_b[lane] = rb;
                     }
                 }
             }
@@ -234,6 +250,7 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
             }
             break;
         }
+        const int ra = S.row_a[lane], rb = S.row_b[lane];
         const bool fresh = S.state[lane] == kNew;
         const int inst = S.inst[lane];
         const double2 *Sb = A.Sbus + (long long)inst * A.sbus_stride;
@@ -270,16 +287,18 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
                 const double sa = S.sa[lane];
                 for (int r = warp; r < n; r += kW) {
                     double2 s = make_double2(0.0, 0.0);
-                    const int p1 = P.Rp[r + 1];
-                    for (int p = P.Rp[r]; p < p1; ++p) {
-                        const double2 y = ybus_lane(P, S, p, lane);
-                        const double2 vv = V[ix(P.Rj[p], lane)];
+                    const int p0 = __ldg(P.Rp + r), p1 = __ldg(P.Rp + r + 1);
+                    const double2 sb = Sb[r];
+                    int c = p0 < p1 ? __ldg(P.Rj + p0) : 0;
+                    for (int p = p0; p < p1; ++p) {
+                        const double2 vv = V[ix(c, lane)];
+                        c = __ldg(P.Rj + min(p + 1, p1 - 1));
+                        const double2 y = ybus_lane(P, S, p, r, lane, ra, rb);
                         s.x += y.x * vv.x - y.y * vv.y;
                         s.y += y.x * vv.y + y.y * vv.x;
                     }
                     Ib[ix(r, lane)] = s;
                     const double2 vr = V[ix(r, lane)];
-                    const double2 sb = Sb[r];
                     double mr = vr.x * s.x + vr.y * s.y - sb.x;
                     const double mi = vr.y * s.x - vr.x * s.y - sb.y;
                     if (P.distributed) mr += sa * P.w[r];
@@ -347,18 +366,23 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
             const bool step = S.state[lane] == kStep;
             // ---- Jacobian values (dS/dVa, |V| dS/d|V|) into the LU array
             if (step) {
+                // the next entry's row and column arrive while this one is worked on
+                int r = warp < P.nnzY ? __ldg(P.Rrow + warp) : 0, c = warp < P.nnzY ? __ldg(P.Rj + warp) : 0;
                 for (int p = warp; p < P.nnzY; p += kW) {
-                    const int r = P.Rrow[p], c = P.Rj[p];
+                    const double2 vr = V[ix(r, lane)], vc = V[ix(c, lane)];
+                    const int4 t = __ldg(P.ytarget + p);
+                    const int q = min(p + kW, P.nnzY - 1);
+                    const int rn = __ldg(P.Rrow + q), cn = __ldg(P.Rj + q);
                     double dvar, dvai;
                     double2 dvm;
-                    const double2 vr = V[ix(r, lane)], vc = V[ix(c, lane)];
-                    dsbus(entry_power(cmul(ybus_lane(P, S, p, lane), vc), vc, vr),
+                    dsbus(entry_power(cmul(ybus_lane(P, S, p, r, lane, ra, rb), vc), vc, vr),
                           r == c ? cmul(cconj(Ib[ix(r, lane)]), vr) : make_double2(0.0, 0.0), dvar, dvai, dvm);
-                    const int4 t = P.ytarget[p];
                     if (t.x >= 0) lu[ix(t.x, lane)] = (LT)dvar;
                     if (t.y >= 0) lu[ix(t.y, lane)] = (LT)dvai;
                     if (t.z >= 0) lu[ix(t.z, lane)] = (LT)dvm.x;
                     if (t.w >= 0) lu[ix(t.w, lane)] = (LT)dvm.y;
+                    r = rn;
+                    c = cn;
                 }
                 for (int i = warp; i < P.nfill; i += kW) lu[ix(P.fillpos[i], lane)] = (LT)0;
                 for (int i = warp; i < P.nconst; i += kW) lu[ix(P.cpos[i], lane)] = (LT)P.cval[i];
@@ -414,9 +438,12 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
                         const int ip = P.xP[r], iq = P.xQ[r];
                         if (ip < 0 && iq < 0) continue;
                         double2 yd = make_double2(0.0, 0.0);
-                        const int p1 = P.Rp[r + 1];
-                        for (int p = P.Rp[r]; p < p1; ++p) {
-                            const double2 y = ybus_lane(P, S, p, lane), d = dV[ix(P.Rj[p], lane)];
+                        const int p0 = __ldg(P.Rp + r), p1 = __ldg(P.Rp + r + 1);
+                        int c = p0 < p1 ? __ldg(P.Rj + p0) : 0;
+                        for (int p = p0; p < p1; ++p) {
+                            const double2 d = dV[ix(c, lane)];
+                            c = __ldg(P.Rj + min(p + 1, p1 - 1));
+                            const double2 y = ybus_lane(P, S, p, r, lane, ra, rb);
                             yd.x += y.x * d.x - y.y * d.y;
                             yd.y += y.x * d.y + y.y * d.x;
                         }
