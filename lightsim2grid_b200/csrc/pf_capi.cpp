@@ -380,6 +380,42 @@ std::vector<int> pack_pairs(const std::vector<int> &a, const std::vector<int> &b
     return out;
 }
 
+// A substitution program of a fast-decoupled system as rows over its constant factors (DevPushes).
+struct PushRows {
+    std::vector<unsigned> idx, mask;
+    std::vector<double> coef;
+    int rows = 0;
+};
+
+void build_push_rows(const l2g::Plan::Program &pr, const std::vector<double> &lu, int m, int threads, PushRows &R) {
+    const unsigned none = (unsigned)m | (unsigned)m << 16;
+    auto add_row = [&]() {
+        R.idx.resize(R.idx.size() + threads, none);
+        R.coef.resize(R.coef.size() + threads, 0.0);
+        if (R.rows % 32 == 0) R.mask.push_back(0u);
+        ++R.rows;
+    };
+    for (int p = 0; p < pr.nphases(); ++p) {
+        const int w = std::max(pr.width[p], 1), n = pr.base[p + 1] - pr.base[p];
+        for (int i = 0; i * w < n; ++i) {
+            add_row();
+            for (int t = 0; t < w && i * w + t < n; ++t) {
+                const int *o = &pr.ops[4 * (size_t)(pr.base[p] + i * w + t)];
+                if (((unsigned)o[3] >> 28) != 2u) continue;  // an empty slot
+                const size_t at = (size_t)(R.rows - 1) * threads + t;
+                R.idx[at] = (unsigned)o[0] | (unsigned)o[2] << 16;
+                R.coef[at] = lu[o[1]] / lu[o[3] & 0x0fffffff];
+            }
+        }
+        if (R.rows > 0) R.mask[(R.rows - 1) / 32] |= 1u << ((R.rows - 1) % 32);
+    }
+    while (R.rows % l2g::kPushAhead) add_row();
+    const int used = R.rows;
+    for (int i = 0; i < l2g::kPushAhead; ++i) add_row();  // loaded ahead, never run
+    R.rows = used;
+    R.mask.push_back(0u);
+}
+
 // The Ybus rows by slots (DevPlan::row_*, off_*, dg_*): host arrays of one plan.
 struct RowSlots {
     int slots = 0, len = 0;
@@ -450,7 +486,7 @@ void build_row_slots(const l2g::Plan &P, RowSlots &R) {
 // Uploads the structure arrays of one plan (and, for a fast-decoupled system, its factor
 // values) into two device blobs and points the fields of `d` into them.
 int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl, const std::vector<double> *luval,
-                int lu_offset = -1, bool compact_ok = true) {
+                int lu_offset = -1, bool compact_ok = true, int threads = 0) {
     std::vector<unsigned char> bi, bd;
     size_t oRp = push(bi, P.Rp), oRj = push(bi, P.Rj), oRrow = push(bi, P.Rrow);
     size_t oyt = push(bi, P.ytarget), oyj = push(bi, P.yjpos);
@@ -514,6 +550,20 @@ int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl,
     size_t oov = push(bd, off), odv = push(bd, dg);
     size_t oRx = push(bd, rx), ow = push(bd, P.weights), ocv = push(bd, P.cval), owJ = push(bd, wJ);
     size_t olu = push(bd, luval ? *luval : std::vector<double>());
+    PushRows push_rows[2];
+    std::vector<double> dval;
+    if (luval) {
+        build_push_rows(P.forward, *luval, P.m, threads, push_rows[0]);
+        build_push_rows(P.backward, *luval, P.m, threads, push_rows[1]);
+        for (int k = 0; k < P.m; ++k) dval.push_back((*luval)[P.dpos[k]]);
+    }
+    size_t opi[2], opm[2], opc[2];
+    for (int k = 0; k < 2; ++k) {
+        opi[k] = push(bi, push_rows[k].idx);
+        opm[k] = push(bi, push_rows[k].mask);
+        opc[k] = push(bd, push_rows[k].coef);
+    }
+    size_t odval = push(bd, dval);
     if (d_int) cudaFree(d_int);
     if (d_dbl) cudaFree(d_dbl);
     d_int = d_dbl = nullptr;
@@ -592,6 +642,10 @@ int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl,
     d.dc = P.dc ? 1 : 0;
     d.slack0 = P.slack0;
     d.luval = luval ? D(olu) : nullptr;
+    for (int k = 0; k < 2; ++k)
+        d.push[k] = l2g::DevPushes{reinterpret_cast<const unsigned *>(bI + opi[k]),
+                                   reinterpret_cast<const unsigned *>(bI + opm[k]), D(opc[k]), push_rows[k].rows};
+    d.dval = D(odval);
     const bool tiled = !P.dc && !P.fdpf;
     d.tfac_ops = tiled ? I4(otfo) : nullptr;
     d.tbwd_ops = tiled ? I4(otbo) : nullptr;
@@ -658,7 +712,7 @@ int upload(pf_plan *pl) {
     l2g::fdpf_lu_offsets(pl->P, off[0], off[1], fits);
     for (int k = 0; k < 2; ++k) {
         rc = upload_plan(pl->P.sub[k], pl->dsub[k], pl->d_sub_int[k], pl->d_sub_dbl[k], &pl->P.sublu[k], off[k],
-                         fits);
+                         fits, pl->threads);
         if (rc) return rc;
     }
     return 0;

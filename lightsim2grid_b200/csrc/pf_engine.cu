@@ -1717,15 +1717,58 @@ __device__ __forceinline__ FdpfLayout fdpf_layout(const DevPlan &P, const DevPla
     return L;
 }
 
+// A substitution program over constant factors: every thread runs its operation of every row (rows are
+// padded, so there is no bounds test), loaded kPushAhead rows ahead and across phases.  The loads are
+// unconditional: one behind a test is merged with the register's old value, which waits for it.
+// The factors' quotients are formed once per plan, so an operation is 12 streamed bytes and one
+// multiply-add; reading both factors and dividing (16-byte operations, a scattered load of each
+// factor, the quotient's chain) N-1 batches took 68.1 ms (2,848 buses, BX) against 27.8 ms now, 1,354 buses
+// 13.2 -> 8.5 ms, 118 buses 1.40 -> 0.51 ms.
+__device__ __forceinline__ void run_pushes(const DevPushes &R, double *v) {
+    constexpr int A = kPushAhead;
+    const unsigned *pi = R.idx + threadIdx.x;
+    const double *pc = R.coef + threadIdx.x;
+    const int bd = blockDim.x, rows = R.rows;
+    unsigned qi[A];
+    double qc[A];
+#pragma unroll
+    for (int i = 0; i < A; ++i) {
+        qi[i] = __ldg(pi + i * bd);
+        qc[i] = __ldg(pc + i * bd);
+    }
+    unsigned m = __ldg(R.mask), mn = __ldg(R.mask + (rows > 32 ? 1 : 0));
+    for (int r = 0; r < rows; r += A) {
+        pi += A * bd;
+        pc += A * bd;
+#pragma unroll
+        for (int i = 0; i < A; ++i) {
+            v[qi[i] & 0xffffu] -= qc[i] * v[qi[i] >> 16];
+            qi[i] = __ldg(pi + i * bd);
+            qc[i] = __ldg(pc + i * bd);
+            if (m & 1u) __syncthreads();
+            m >>= 1;
+        }
+        if (((r + A) & 31) == 0) {
+            m = mn;
+            mn = __ldg(R.mask + min((r + A) / 32 + 1, rows / 32));
+        }
+    }
+}
+
 // B x = b for one decoupled system: forward and backward programs over the constant factors,
 // then the division by the pivots (the backward program keeps z undivided).
 template <bool LU_SMEM>
 __device__ __forceinline__ void fdpf_solve(const DevPlan &B, const FdpfLayout &L, int k, Trace &tr) {
     double *x = L.x[k];
-    double *lu = const_cast<double *>(L.lu[k]);  // read only: substitutions do not write the LU
-    run_lu_program<double, double, LU_SMEM>(B.fwd_cops, B.fwd_ops, L.sbf[k], L.swf[k], B.fwd_nph, B.m, lu, x, tr);
-    run_lu_program<double, double, LU_SMEM>(B.bwd_cops, B.bwd_ops, L.sbb[k], L.swb[k], B.bwd_nph, B.m, lu, x, tr);
-    for (int i = threadIdx.x; i < B.m; i += blockDim.x) x[i] = x[i] / lu[B.dpos[i]];
+    if constexpr (LU_SMEM) {
+        double *lu = const_cast<double *>(L.lu[k]);  // read only: substitutions do not write the LU
+        run_lu_program<double, double, true>(B.fwd_cops, B.fwd_ops, L.sbf[k], L.swf[k], B.fwd_nph, B.m, lu, x, tr);
+        run_lu_program<double, double, true>(B.bwd_cops, B.bwd_ops, L.sbb[k], L.swb[k], B.bwd_nph, B.m, lu, x, tr);
+    } else {
+        run_pushes(B.push[0], x);
+        run_pushes(B.push[1], x);
+    }
+    for (int i = threadIdx.x; i < B.m; i += blockDim.x) x[i] = lu_div(x[i], __ldg(B.dval + i));
     __syncthreads();
 }
 
@@ -1747,8 +1790,8 @@ __device__ void fdpf_mismatch(const DevPlan &P, Shared &S, const double2 *__rest
         double mi = vr.y * s.x - vr.x * s.y - sb.y;
         mr += sa * P.w[r];
         const double vm = Vm[r];
-        mr /= vm;
-        mi /= vm;
+        mr = lu_div(mr, vm);
+        mi = lu_div(mi, vm);
         lbad |= !isfinite(mr) || !isfinite(mi);
         const int ip = P.dg_eq[slot].x, iq = P.dg_eq[slot].y;
         if (ip >= 0) {
@@ -1792,6 +1835,8 @@ __global__ void __launch_bounds__(MAXT, MINB) fdpf_batch_kernel(const DevPlan P0
             for (int i = tid; i < b.bwd_nph; i += blockDim.x) L.swb[k][i] = b.bwd_width[i];
             if (LU_SMEM)
                 for (int i = tid; i < b.nnzLU; i += blockDim.x) L.x[k][b.lu_offset + i] = b.luval[i];
+            else if (tid == 0)
+                L.x[k][b.m] = 0.0;  // the padding operations' element (later any value of the other system)
         }
     }
     __syncthreads();
@@ -1872,8 +1917,12 @@ __global__ void __launch_bounds__(MAXT, MINB) fdpf_batch_kernel(const DevPlan P0
                     const double vm = Vm[b];
                     const double2 v = make_double2(vm * cs, vm * sn);
                     V[b] = v;
-                    Vm[b] = cabs2(v);
-                    Va[b] = atan2(v.y, v.x);
+                    // |V| and arg(V) only where they differ from the updated values (voltage_update)
+                    if (!(vm >= 0.0 && fabs(va) <= kPi)) {
+                        Vm[b] = cabs2(v);
+                        va = atan2(v.y, v.x);
+                    }
+                    Va[b] = va;
                 }
                 __syncthreads();
                 fdpf_mismatch(P, S, V, Vm, Sb, L.x[0], 1, norm, bad);
@@ -1894,8 +1943,11 @@ __global__ void __launch_bounds__(MAXT, MINB) fdpf_batch_kernel(const DevPlan P0
                     const double2 t = T[b];
                     const double2 v = make_double2(vm * t.x, vm * t.y);
                     V[b] = v;
-                    Vm[b] = cabs2(v);
-                    Va[b] = atan2(v.y, v.x);
+                    if (!(vm >= 0.0)) {  // negative (or not finite): re-derived, with the angle turned
+                        vm = cabs2(v);
+                        Va[b] = atan2(v.y, v.x);
+                    }
+                    Vm[b] = vm;
                 }
                 __syncthreads();
                 fdpf_mismatch(P, S, V, Vm, Sb, L.x[0], 0, norm, bad);

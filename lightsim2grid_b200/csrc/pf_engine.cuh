@@ -8,6 +8,16 @@
 
 namespace l2g {
 
+// A substitution program over constant factors (fast decoupled systems): rows of `threads` operations
+// v[x] -= coef * v[z], x | z << 16 in idx, padded with operations on the scratch element m; bit r of
+// mask: a barrier after row r.  rows is a multiple of kPushAhead; as many rows of padding follow.
+struct DevPushes {
+    const unsigned *idx, *mask;
+    const double *coef;
+    int rows;
+};
+constexpr int kPushAhead = 4;
+
 // Structure arrays of one plan on the device (see pf_plan.hpp for their meaning).
 struct DevPlan {
     int n, m, nnzY, nnzLU, distributed;
@@ -58,6 +68,8 @@ struct DevPlan {
     const int *dpos;         // pivot position per column (m)
     int dc, slack0;          // DC plan (B = Re(Ybus) without the slack) and its slack bus
     const double *luval;     // constant factor values (LU layout) of a fast-decoupled system
+    DevPushes push[2];       // ... its forward and backward programs over them
+    const double *dval;      // ... its pivots (m)
     // the phase programs regrouped for the batch-interleaved kernel (TileProgram, pf_plan.hpp):
     // operations (kind 7 padding) and, per phase, the first chunk and the number of rounds
     const int4 *tfac_ops, *tbwd_ops, *tfwd_ops;
