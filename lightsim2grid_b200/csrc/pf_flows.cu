@@ -21,6 +21,7 @@
 namespace l2g {
 namespace {
 
+
 __device__ __forceinline__ double2 cmulf(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -32,43 +33,57 @@ __device__ __forceinline__ int source_row(const FlowArgs &A, int r) {
     return src;
 }
 
-// Flows of one branch at one row's voltages ef (from) and et (to).
-__device__ __forceinline__ void branch_flow(double2 yf, double2 yt, double vn, double sn, double2 ef, double2 et,
+// Flows of one branch at one row's voltages ef (from) and et (to); ka = sn_mva / (sqrt(3) vn).  The
+// reference divides |E_f I_ft| by |E_f|, which leaves |I_ft| (one square root instead of two and a
+// division: FP64 arithmetic was a third of the time); a zero or non-finite E_f gives the NaN of that
+// quotient.
+__device__ __forceinline__ void branch_flow(double2 yf, double2 yt, double ka, double sn, double2 ef, double2 et,
                                             double &a, double &p) {
-    const double sqrt3 = 1.7320508075688772;
     const double2 i1 = cmulf(yf, ef), i2 = cmulf(yt, et);
     const double2 ift = make_double2(i1.x + i2.x, -(i1.y + i2.y));  // conj
-    const double2 s = cmulf(ef, ift);
-    const double vf_kv = sqrt(ef.x * ef.x + ef.y * ef.y) * vn;
-    a = sqrt(s.x * s.x + s.y * s.y) * sn / (sqrt3 * vf_kv);
-    p = s.x * sn;
+    const double e2 = ef.x * ef.x + ef.y * ef.y;
+    a = sqrt(ift.x * ift.x + ift.y * ift.y) * ka;
+    if (!(e2 > 0.0 && isfinite(e2))) a = nan("");
+    p = (ef.x * ift.x - ef.y * ift.y) * sn;
 }
 
-// One CTA per row (grid-stride over rows); each thread takes every blockDim-th branch and
-// gathers its two voltages through L1 (a row's voltages stay cached while the CTA works on it).
-// Measured on the 2848-bus N-1 flows (3776 x 3776): 0.18 ms; staging the row, or tiles of rows,
-// in shared memory was slower (0.19 / 0.27 ms: fewer CTAs per SM in flight).
-__global__ void __launch_bounds__(256) branch_flows_kernel(const FlowArgs A) {
+__device__ __forceinline__ double amps_factor(double sn, double vn) { return sn / (1.7320508075688772 * vn); }
+
+// One CTA per row (grid-stride over rows); each thread takes every NT-th branch and gathers its two
+// voltages through L1.  Bound by those random 16-byte gathers: the rows in work on an SM have to stay in
+// its L1.  So rows of kWideRow bytes and more run two CTAs of 1024 threads per SM, smaller ones six of
+// 256 (and 40 registers).  2848 buses, 3776 rows: 188 us with eight CTAs of 256 and two square
+// roots and a division per flow, 138 us with six CTAs and one root, 122 us with the two wide CTAs; 300
+// buses, 4000 rows: 19.9 -> 16.9 us (wide CTAs: 23.3).  Two or four rows per CTA (branch data read once
+// for all) and tiles of rows staged in shared memory were slower (127-300 and 143 us).
+constexpr size_t kWideRow = 24000;
+template <int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) branch_flows_kernel(const FlowArgs A) {
     for (int row = blockIdx.x; row < A.nrows; row += gridDim.x) {
         const int src = source_row(A, row);
         const double2 *V = src >= 0 ? A.V + (long long)src * A.v_stride : nullptr;
         const int o0 = A.out_ptr ? A.out_ptr[row] : 0, o1 = A.out_ptr ? A.out_ptr[row + 1] : 0;
-        for (int k = threadIdx.x; k < A.nbr; k += blockDim.x) {
+        const int first = o0 < o1 ? A.out_ids[o0] : -1;
+        for (int k = threadIdx.x; k < A.nbr; k += NT) {
             double a = 0.0, p = 0.0;
-            if (A.status == nullptr || A.status[k]) {
-                const int f = A.from[k], t = A.to[k];
-                const double2 ef = V ? V[f] : make_double2(0.0, 0.0);
-                const double2 et = V ? V[t] : make_double2(0.0, 0.0);
-                branch_flow(A.yff[k], A.yft[k], A.vn_kv_from[k], A.sn_mva, ef, et, a, p);
+            if (A.status == nullptr || __ldg(A.status + k)) {
+                const int f = __ldg(A.from + k), t = __ldg(A.to + k);
+                const double2 yf = __ldg(A.yff + k), yt = __ldg(A.yft + k);
+                const double ka = A.amps ? amps_factor(A.sn_mva, __ldg(A.vn_kv_from + k)) : 0.0;
+                const double2 ef = V ? __ldg(V + f) : make_double2(0.0, 0.0);
+                const double2 et = V ? __ldg(V + t) : make_double2(0.0, 0.0);
+                branch_flow(yf, yt, ka, A.sn_mva, ef, et, a, p);
             }
             // clean_flows: the branches removed in this row's case are 0 where finite
-            for (int o = o0; o < o1; ++o)
-                if (A.out_ids[o] == k) {
-                    if (isfinite(a)) a = 0.0;
-                    if (isfinite(p)) p = 0.0;
-                }
-            if (A.amps) A.amps[(long long)row * A.nbr + k] = a;
-            if (A.p_mw) A.p_mw[(long long)row * A.nbr + k] = p;
+            bool out = first == k;
+            for (int o = o0 + 1; o < o1; ++o) out |= A.out_ids[o] == k;
+            if (out) {
+                if (isfinite(a)) a = 0.0;
+                if (isfinite(p)) p = 0.0;
+            }
+            const long long at = (long long)row * A.nbr + k;
+            if (A.amps) __stcs(A.amps + at, a);
+            if (A.p_mw) __stcs(A.p_mw + at, p);
         }
     }
 }
@@ -77,7 +92,10 @@ __global__ void __launch_bounds__(256) branch_flows_kernel(const FlowArgs A) {
 
 cudaError_t launch_branch_flows(const FlowArgs &A, int num_sms, cudaStream_t st) {
     if (A.nrows <= 0 || A.nbr <= 0) return cudaSuccess;
-    branch_flows_kernel<<<std::min(A.nrows, num_sms * 8), 256, 0, st>>>(A);
+    if ((size_t)A.n * sizeof(double2) >= kWideRow)
+        branch_flows_kernel<1024, 2><<<std::min(A.nrows, num_sms * 2), 1024, 0, st>>>(A);
+    else
+        branch_flows_kernel<256, 6><<<std::min(A.nrows, num_sms * 6), 256, 0, st>>>(A);
     return cudaGetLastError();
 }
 
