@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cstring>
 #include <functional>
+#include <map>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -628,6 +629,7 @@ int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl,
     auto U2 = [&](size_t o) { return reinterpret_cast<const uint2 *>(bI + o); };
     d.compact = compact ? 1 : 0;
     d.lu_offset = lu_offset >= 0 ? lu_offset : l2g::compact_lu_offset(P.m);
+    d.cops_runs = compact && lu_offset < 0 && P.bank_lanes == 0 ? 1 : 0;
     d.fac_cops = compact ? U2(ocf) : nullptr;
     d.bwd_cops = compact ? U2(ocb) : nullptr;
     d.fwd_cops = compact ? U2(ocw) : nullptr;
@@ -2163,6 +2165,29 @@ int pf_host_schedule_solve(int n, const int *colptr, const int *rowind, const do
         }
     };
     const std::vector<double> lu0 = lu, xs0 = xs;
+    // what the global-memory LU kernel assumes of a phase: the operations that write one value follow one
+    // another on their thread, and no operation reads a value that another one of the phase writes
+    for (const l2g::Plan::Program *pr : {&P.factor, &P.backward, &P.forward})
+        for (int p = 0; p < pr->nphases(); ++p) {
+            std::map<std::pair<int, int>, int> run;  // written value -> its last operation
+            const int b = pr->base[p], w = pr->width[p], e = pr->base[p + 1];
+            for (int t = 0; t < w; ++t)
+                for (int o = b + t; o < e; o += w) {
+                    const int kind = (unsigned)pr->ops[4 * o + 3] >> 28;
+                    if (kind == 7) continue;
+                    auto it = run.emplace(std::make_pair(kind, pr->ops[4 * o]), o).first;
+                    if (it->second != o && it->second != o - w)
+                        return fail(-1, "schedule check: a value's operations do not follow one another");
+                    it->second = o;
+                }
+            for (int o = b; o < e; ++o) {
+                const int kind = (unsigned)pr->ops[4 * o + 3] >> 28;
+                if (kind == 7) continue;
+                if (run.count({0, pr->ops[4 * o + 1]}) || run.count({kind, pr->ops[4 * o + 2]}) ||
+                    run.count({0, pr->ops[4 * o + 3] & 0x0fffffff}))
+                    return fail(-1, "schedule check: an operation reads a value written in its phase");
+            }
+        }
     // the bank-conflict placement of the packed programs gives the same bits: every written
     // value keeps its thread and the order of its operations.  Checked for the placement of this
     // plan (4-byte words), for the one built for 8-byte words (FP64) and for the spread clusters.

@@ -354,11 +354,6 @@ struct OpPair {
 };
 
 template <typename OP>
-__device__ __forceinline__ OP empty_op();
-template <>
-__device__ __forceinline__ int4 empty_op<int4>() { return make_int4(0, 0, 0, 7 << 28); }
-
-template <typename OP>
 __device__ __forceinline__ void load_first2(const OP *__restrict__ ops, const int *sb, const int *sw, int nph,
                                             int p, OpPair<OP> &r, OP none) {
     r.a = none;
@@ -462,13 +457,178 @@ __device__ void run_program_narrow(const OP *__restrict__ ops, const int *sb, co
     }
 }
 
+// An operation of a program over an LU in global memory, decoded: the written value x and an `id` that
+// is distinct for every written value, the operands' LU positions y and w, and z.  A push writes and
+// reads (x, z) the solve vector, an update the LU.
+struct GlobalOp {
+    unsigned x, y, z, w, id;
+    bool none, push;
+};
+__device__ __forceinline__ GlobalOp decode(const int4 o, int, int) {
+    const unsigned kind = (unsigned)o.w >> 28;
+    return GlobalOp{(unsigned)o.x, (unsigned)o.y, (unsigned)o.z, (unsigned)o.w & 0x0fffffffu,
+                    (unsigned)o.x | (kind << 28), kind == 7u, kind == 2u};
+}
+// packed: solve vector below `off`, LU from there on; m: the scratch element of an empty slot
+__device__ __forceinline__ GlobalOp decode(const uint2 o, int m, int off) {
+    const unsigned X = o.x & 0xffffu, Z = o.y & 0xffffu;
+    const bool push = X < (unsigned)off;
+    const unsigned d = push ? 0u : (unsigned)off;
+    return GlobalOp{X - d, (o.x >> 16) - off, Z - d, (o.y >> 16) - off, X, X == (unsigned)m, push};
+}
+__device__ __forceinline__ uint2 none_op(uint2, int m) {
+    return make_uint2((unsigned)m | ((unsigned)m << 16), (unsigned)m | ((unsigned)m << 16));
+}
+__device__ __forceinline__ int4 none_op(int4, int) { return make_int4(0, 0, 0, 7 << 28); }
+
+// Runs a phase program over an LU in global memory, the solve vector in shared memory: in phase p,
+// thread t < sw[p] runs the operations sb[p] + t, sb[p] + t + sw[p], ... in order, one barrier per phase.
+// Bound by the latency of its scattered loads from L2: one operation after the other, each waited for the
+// store of the one before.  So a thread takes U operations together (no operation reads a value that
+// another one of its phase writes, and those that write one value follow one another on their thread:
+// their sum stays in a register), the next U arriving meanwhile, in the packed form where 16-bit
+// indices hold the LU (half the bytes: 2.4 MB of operations were read per factorisation).  2848 buses
+// FP64, N-1, 3,050 outages: 14.7 -> 13.2 ms with run_pushes_global (U = 2, 4: 14.2, 13.8 ms; U = 6 and 8 spill:
+// 16.7, 23.2 ms before run_pushes_global; operation loads past L1: +0.4 ms).  16-byte operations run U = 2
+// (300-chord grid FP64 93.5 -> 91.0 ms).  FP32 keeps one operation at a time (run_program: 51.9 ms on the 300-chord
+// grid against 55.4).
+// A function of its own: inlined it spilled in the Newton loop.
+template <int U, typename OP, typename T>
+__device__ __noinline__ void run_program_global(const OP *__restrict__ ops, const int *sb, const int *sw, int nph,
+                                                int m, int off, T *lu, T *x, Trace &tr) {
+    if (nph <= 0) return;
+    const int t = threadIdx.x;
+    const auto load = [&](OP (&o)[U], int k, int w, int e) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) o[u] = k + u * w < e ? __ldg(ops + k + u * w) : none_op(OP{}, m);
+    };
+    OP o[U], n[U];
+    int w = sw[0], e = sb[1], k = t < w ? sb[0] + t : e;
+    load(o, k, w, e);
+    for (int p = 0;;) {
+        T y[U], d[U], z[U], v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const GlobalOp g = decode(o[u], m, off);
+            y[u] = d[u] = z[u] = v[u] = (T)1;
+            if (!g.none) {
+                const T *s = g.push ? x : lu;
+                y[u] = lu[g.y];
+                d[u] = lu[g.w];
+                z[u] = s[g.z];
+                if (u == 0 || g.id != decode(o[u > 0 ? u - 1 : 0], m, off).id) v[u] = s[g.x];
+            }
+        }
+        // the next operations: of this phase, else the first of the next one
+        k += U * w;
+        const bool last = k >= e;
+        if (last) {
+            k = e = 0;
+            if (p + 1 < nph) {
+                w = sw[p + 1];
+                e = sb[p + 2];
+                k = t < w ? sb[p + 1] + t : e;
+            }
+        }
+        load(n, k, w, e);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const GlobalOp g = decode(o[u], m, off);
+            if (g.none) continue;
+            if (u > 0 && g.id == decode(o[u > 0 ? u - 1 : 0], m, off).id) v[u] = v[u > 0 ? u - 1 : 0];
+            const T q = lu_div(g.push ? y[u] * z[u] : z[u], d[u]);
+            v[u] -= g.push ? q : y[u] * q;
+            if (u == U - 1 || g.id != decode(o[u < U - 1 ? u + 1 : u], m, off).id) (g.push ? x : lu)[g.x] = v[u];
+        }
+        if (last) {
+            __syncthreads();
+            tr.mark();
+            if (++p >= nph) break;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) o[u] = n[u];
+    }
+}
+
+// A substitution program (pushes only) over an LU in global memory.  A phase waited for its operands from L2
+// after its barrier; but the LU is final here, so a thread's LU values for its next U operations are loaded
+// while the current ones run, and their operations one batch earlier still.  N-1: 2848 buses FP64 backward
+// 111k -> 98k SM cycles a Newton step (with packed operations), 300-chord grid mixed 51.9 -> 50.1 ms (U = 1:
+// 50.9 ms).
+template <int U, typename OP, typename T>
+__device__ __noinline__ void run_pushes_global(const OP *__restrict__ ops, const int *sb, const int *sw, int nph,
+                                               int m, int off, const T *lu, T *x, Trace &tr) {
+    if (nph <= 0) return;
+    const int t = threadIdx.x;
+    int p = 0, w = sw[0], e = sb[1], k = t < w ? sb[0] + t : e;  // the batch loaded next
+    // loads a batch and moves on; whether it is its phase's last one
+    const auto load = [&](OP (&o)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) o[u] = k + u * w < e ? __ldg(ops + k + u * w) : none_op(OP{}, m);
+        k += U * w;
+        const bool last = k >= e;
+        if (last) {
+            k = e = 0;
+            if (++p < nph) {
+                w = sw[p];
+                e = sb[p + 1];
+                k = t < w ? sb[p] + t : e;
+            }
+        }
+        return last;
+    };
+    const auto values = [&](const OP (&o)[U], T (&y)[U], T (&d)[U]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const GlobalOp g = decode(o[u], m, off);
+            y[u] = g.none ? (T)0 : lu[g.y];
+            d[u] = g.none ? (T)1 : lu[g.w];
+        }
+    };
+    OP o[U], n[U], nn[U];
+    T y[U], d[U], yn[U], dn[U];
+    bool last = load(o), lastn = load(n);
+    values(o, y, d);
+    for (int left = nph;;) {
+        values(n, yn, dn);
+        const bool lastnn = load(nn);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const GlobalOp g = decode(o[u], m, off);
+            if (!g.none) x[g.x] -= lu_div(y[u] * x[g.z], d[u]);
+        }
+        if (last) {
+            __syncthreads();
+            tr.mark();
+            if (--left == 0) break;
+        }
+        last = lastn;
+        lastn = lastnn;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            o[u] = n[u];
+            n[u] = nn[u];
+            y[u] = yn[u];
+            d[u] = dn[u];
+        }
+    }
+}
+
+// The packed operations where a kernel variant can run them: an LU in global memory takes those whose
+// placement keeps a value's operations together (null: the int4 ones).
+template <bool LU_SMEM>
+__device__ __forceinline__ const uint2 *packed_ops(const DevPlan &P, const uint2 *cops) {
+    return LU_SMEM || P.cops_runs ? cops : nullptr;
+}
+
 // One program over the LU layout of the kernel variant: packed operations over the shared
-// index space, or int4 operations over the global LU and the shared solve vector.
+// index space, or packed or int4 operations over the global LU and the shared solve vector.
+// PUSH: a substitution program.
 // NARROW: `nar` is the narrow range of this program (phases [nar.x, nar.y) on nar.z warps,
 // operations staged at `sops`), packed layout only.
-template <typename LT, typename XT, bool LU_SMEM, bool NARROW = false>
+template <typename LT, typename XT, bool LU_SMEM, bool PUSH, bool NARROW = false>
 __device__ __forceinline__ void run_lu_program(const uint2 *cops, const int4 *ops, const int *sb, const int *sw,
-                                               int nph, int m, LT *lu, XT *x, Trace &tr,
+                                               int nph, int m, int off, LT *lu, XT *x, Trace &tr,
                                                int3 nar = make_int3(0, 0, 0), const uint2 *sops = nullptr) {
     if constexpr (LU_SMEM) {
         static_assert(sizeof(LT) == sizeof(XT), "the packed layout needs one element type");
@@ -479,8 +639,17 @@ __device__ __forceinline__ void run_lu_program(const uint2 *cops, const int4 *op
         else
             run_program<uint2>(cops, sb, sw, nph, none, [x](const uint2 o) { run_op_packed<XT>(o, x); }, tr);
     } else {
-        run_program<int4>(ops, sb, sw, nph, empty_op<int4>(), [lu, x](const int4 o) { run_op<LT, XT>(o, lu, x); },
-                          tr);
+        static_assert(sizeof(LT) == sizeof(XT), "one element type");
+        if constexpr (PUSH) {
+            if (cops != nullptr) run_pushes_global<2, uint2, XT>(cops, sb, sw, nph, m, off, lu, x, tr);
+            else run_pushes_global<2, int4, XT>(ops, sb, sw, nph, m, 0, lu, x, tr);
+        } else if constexpr (sizeof(LT) == 8) {
+            if (cops != nullptr) run_program_global<3, uint2, XT>(cops, sb, sw, nph, m, off, lu, x, tr);
+            else run_program_global<2, int4, XT>(ops, sb, sw, nph, m, 0, lu, x, tr);
+        } else {
+            run_program<int4>(ops, sb, sw, nph, none_op(int4{}, 0), [lu, x](const int4 o) { run_op<LT, XT>(o, lu, x); },
+                              tr);
+        }
     }
 }
 
@@ -1268,18 +1437,21 @@ __device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, 
         pr.traced = 1;
         const auto program_factor = [&]() {
             const Layout<LT, XT> L = lay();
-            run_lu_program<LT, XT, LU_SMEM, NARROW>(P.fac_cops, P.fac_ops, L.sb_fac, L.sw_fac, P.fac_nph, m, L.lu, x,
-                                                    tr, make_int3(P.nar_a[0], P.nar_b[0], P.nar_warps), L.nar_ops[0]);
+            run_lu_program<LT, XT, LU_SMEM, false, NARROW>(packed_ops<LU_SMEM>(P, P.fac_cops), P.fac_ops, L.sb_fac, L.sw_fac,
+                                                          P.fac_nph, m, P.lu_offset, L.lu, x, tr,
+                                                          make_int3(P.nar_a[0], P.nar_b[0], P.nar_warps), L.nar_ops[0]);
         };
         const auto program_backward = [&]() {
             const Layout<LT, XT> L = lay();
-            run_lu_program<LT, XT, LU_SMEM, NARROW>(P.bwd_cops, P.bwd_ops, L.sb_bwd, L.sw_bwd, P.bwd_nph, m, L.lu, x,
-                                                    tr, make_int3(P.nar_a[1], P.nar_b[1], P.nar_warps), L.nar_ops[1]);
+            run_lu_program<LT, XT, LU_SMEM, true, NARROW>(packed_ops<LU_SMEM>(P, P.bwd_cops), P.bwd_ops, L.sb_bwd, L.sw_bwd,
+                                                          P.bwd_nph, m, P.lu_offset, L.lu, x, tr,
+                                                          make_int3(P.nar_a[1], P.nar_b[1], P.nar_warps), L.nar_ops[1]);
         };
         const auto program_forward = [&]() {
             const Layout<LT, XT> L = lay();
-            run_lu_program<LT, XT, LU_SMEM, NARROW>(P.fwd_cops, P.fwd_ops, L.sb_fwd, L.sw_fwd, P.fwd_nph, m, L.lu, x,
-                                                    tr, make_int3(P.nar_a[2], P.nar_b[2], P.nar_warps), L.nar_ops[2]);
+            run_lu_program<LT, XT, LU_SMEM, true, NARROW>(packed_ops<LU_SMEM>(P, P.fwd_cops), P.fwd_ops, L.sb_fwd, L.sw_fwd,
+                                                          P.fwd_nph, m, P.lu_offset, L.lu, x, tr,
+                                                          make_int3(P.nar_a[2], P.nar_b[2], P.nar_warps), L.nar_ops[2]);
         };
         bool have_lu = false;  // this instance's LU from an earlier iteration is in place
         while (!conv && it < A.max_iter) {
@@ -1612,15 +1784,15 @@ __global__ void __launch_bounds__(512, 1) dc_batch_kernel(const DevPlan P, const
                 if (ip >= 0) x[ip] = Sb[b].x;
             }
             __syncthreads();
-            run_lu_program<double, double, LU_SMEM>(P.fac_cops, P.fac_ops, L.sb_fac, L.sw_fac, P.fac_nph, m, lu, x,
-                                                    tr);
+            run_lu_program<double, double, LU_SMEM, false>(packed_ops<LU_SMEM>(P, P.fac_cops), P.fac_ops, L.sb_fac, L.sw_fac,
+                                                           P.fac_nph, m, P.lu_offset, lu, x, tr);
             check_pivots<double>(P, S, lu);
             int err = 0;
             if (S.piv_err) {
                 err = 6;  // SolverReFactor
             } else {
-                run_lu_program<double, double, LU_SMEM>(P.bwd_cops, P.bwd_ops, L.sb_bwd, L.sw_bwd, P.bwd_nph, m, lu,
-                                                        x, tr);
+                run_lu_program<double, double, LU_SMEM, true>(packed_ops<LU_SMEM>(P, P.bwd_cops), P.bwd_ops, L.sb_bwd,
+                                                              L.sw_bwd, P.bwd_nph, m, P.lu_offset, lu, x, tr);
                 scale_by_pivots<double, double>(P, S, lu, x);
                 double lmax = 0.0;
                 int lbad = 0;
@@ -1762,8 +1934,10 @@ __device__ __forceinline__ void fdpf_solve(const DevPlan &B, const FdpfLayout &L
     double *x = L.x[k];
     if constexpr (LU_SMEM) {
         double *lu = const_cast<double *>(L.lu[k]);  // read only: substitutions do not write the LU
-        run_lu_program<double, double, true>(B.fwd_cops, B.fwd_ops, L.sbf[k], L.swf[k], B.fwd_nph, B.m, lu, x, tr);
-        run_lu_program<double, double, true>(B.bwd_cops, B.bwd_ops, L.sbb[k], L.swb[k], B.bwd_nph, B.m, lu, x, tr);
+        run_lu_program<double, double, true, true>(B.fwd_cops, B.fwd_ops, L.sbf[k], L.swf[k], B.fwd_nph, B.m, B.lu_offset,
+                                                   lu, x, tr);
+        run_lu_program<double, double, true, true>(B.bwd_cops, B.bwd_ops, L.sbb[k], L.swb[k], B.bwd_nph, B.m, B.lu_offset,
+                                                   lu, x, tr);
     } else {
         run_pushes(B.push[0], x);
         run_pushes(B.push[1], x);

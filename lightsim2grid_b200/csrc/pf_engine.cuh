@@ -58,6 +58,7 @@ struct DevPlan {
     int fac_nph, bwd_nph, fwd_nph;
     // packed operations of the shared-memory layout (x and LU in one index space)
     int compact, lu_offset;
+    int cops_runs;           // their operations that write one value follow one another on their thread
     const uint2 *fac_cops, *bwd_cops, *fwd_cops;
     // narrow phases of the packed programs (shared-memory LU): phases [nar_a[k], nar_b[k]) of
     // program k (0 factor, 1 backward, 2 forward) run on the first nar_warps warps only, between
