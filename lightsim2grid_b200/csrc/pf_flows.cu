@@ -51,12 +51,15 @@ __device__ __forceinline__ double amps_factor(double sn, double vn) { return sn 
 
 // One CTA per row (grid-stride over rows); each thread takes every NT-th branch and gathers its two
 // voltages through L1.  Bound by those random 16-byte gathers: the rows in work on an SM have to stay in
-// its L1.  So rows of kWideRow bytes and more run two CTAs of 1024 threads per SM, smaller ones six of
-// 256 (and 40 registers).  2848 buses, 3776 rows: 188 us with eight CTAs of 256 and two square
+// its L1.  So rows of which six do not fit it (kWideRow) run two CTAs of 1024 threads per SM, smaller ones six
+// of 256 (and 40 registers): 2848 buses, 3776 rows: 188 us with eight CTAs of 256 and two square
 // roots and a division per flow, 138 us with six CTAs and one root, 122 us with the two wide CTAs; 300
-// buses, 4000 rows: 19.9 -> 16.9 us (wide CTAs: 23.3).  Two or four rows per CTA (branch data read once
+// buses, 4000 rows: 19.9 -> 16.9 us (wide CTAs: 23.3); 1600 and 2000 buses, 4000 rows: six narrow CTAs 84 and
+// 104 us, two wide ones 100 and 114, at 2200 the same.  Few rows are spread over more threads: with at most as
+// many rows as wide CTAs run at once (30 rows of 1200 buses: 16.4 -> 12.3 us), or twice as many where a narrow
+// CTA takes long (320 rows of 2000 buses: 20.5 against 24.6 us).  Two or four rows per CTA (branch data read once
 // for all) and tiles of rows staged in shared memory were slower (127-300 and 143 us).
-constexpr size_t kWideRow = 24000;
+constexpr size_t kWideRow = 34000, kLongRow = 24000;
 template <int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) branch_flows_kernel(const FlowArgs A) {
     for (int row = blockIdx.x; row < A.nrows; row += gridDim.x) {
@@ -92,7 +95,9 @@ __global__ void __launch_bounds__(NT, MINB) branch_flows_kernel(const FlowArgs A
 
 cudaError_t launch_branch_flows(const FlowArgs &A, int num_sms, cudaStream_t st) {
     if (A.nrows <= 0 || A.nbr <= 0) return cudaSuccess;
-    if ((size_t)A.n * sizeof(double2) >= kWideRow)
+    const size_t row = (size_t)A.n * sizeof(double2);
+    const bool few = A.nbr > 512 && A.nrows <= (row >= kLongRow ? 4 : 2) * num_sms;
+    if (few || row >= kWideRow)
         branch_flows_kernel<1024, 2><<<std::min(A.nrows, num_sms * 2), 1024, 0, st>>>(A);
     else
         branch_flows_kernel<256, 6><<<std::min(A.nrows, num_sms * 6), 256, 0, st>>>(A);
