@@ -140,12 +140,14 @@ __device__ __forceinline__ double2 ybus_value(const DevPlan &P, const Shared &S,
 }
 
 
-// Stages override i of an instance (caller: one thread per override).
+// Stages override i of an instance (caller: one thread per override).  A position outside the pattern
+// (pf_ybus_positions gives -1 there) changes no entry.
 __device__ __forceinline__ void stage_override(const DevPlan &P, Shared &S, int i, int pos, double2 val) {
+    const bool in = (unsigned)pos < (unsigned)P.nnzY;
     S.opos[i] = pos;
     S.oval[i] = val;
-    S.orow[i] = P.Rrow[pos];
-    S.ocol[i] = P.Rj[pos];
+    S.orow[i] = in ? P.Rrow[pos] : -1;
+    S.ocol[i] = in ? P.Rj[pos] : -1;
 }
 
 // The overrides that lie in row r, as a bit mask: rows without one (nearly all) then test nothing

@@ -205,9 +205,11 @@ __global__ void __launch_bounds__(1024, 1) nr_tile_kernel(const DevPlan P, const
                         S.novr[lane] = k1 - k0;
                         int ra = -1, rb = -1;
                         for (int i = 0; i < k1 - k0; ++i) {
-                            const int pos = A.ovr_pos[k0 + i], r = P.Rrow[pos];
+                            const int pos = A.ovr_pos[k0 + i];
                             S.opos[i][lane] = pos;
                             S.oval[i][lane] = A.ovr_val[k0 + i];
+                            if ((unsigned)pos >= (unsigned)P.nnzY) continue;  // outside the pattern: no entry
+                            const int r = P.Rrow[pos];
                             if (ra == -1 || r == ra) ra = r;
                             else if (rb == -1 || r == rb) rb = r;
                             else ra = -2;
