@@ -316,7 +316,9 @@ int pf_flows_host(const pf_branch_set *br, int n, int nrows, const double *V_ri,
    cptr[p+1]), each 4 * branch + kind (0 ff, 1 tt, 2 ft, 3 tf), computed from the branch's r,
    x, total shunt h (complex, split half / half) and in-service flag (NULL: all in service).
    pf_set_ybus_values_device copies such values (the plan's storage order) into the plan's
-   device Ybus, asynchronously: later launches on the plan use them.  The plan's host-side
+   device Ybus, asynchronously: later launches on the plan use them.  The values may be any device
+   memory (8-byte aligned) and the stream any device's; with another device's stream than the plan's the
+   call returns when the values are in place.  The plan's host-side
    values (pf_n1_prepare's islanding check, pf_get_J) keep what pf_plan_create or
    pf_set_ybus_values gave. */
 int pf_ybus_positions(const pf_plan *plan, int ncoef, const int *rows, const int *cols, int *pos);
@@ -449,6 +451,12 @@ int pf_host_schedule_solve(int n, const int *colptr, const int *rowind, const do
                            const double *V_ri, const int *slack_ids, int nslack, const double *slack_weights,
                            const int *pv, int npv, const int *pq, int npq, int distributed, const double *b,
                            double *x, pf_plan_info *info);
+
+/* How pf_set_ybus_values_device takes a source at address `source` on source_device (-1: not device
+   memory) with a stream of stream_device: 0 the plan's kernel reads it on the stream, 1 it is copied into
+   the plan first, 2 (a stream of another device than the plan's) copied on the stream, then the kernel on
+   the plan's device. */
+int pf_host_ybus_route(int plan_device, int stream_device, int source_device, unsigned long long source);
 
 #ifdef __cplusplus
 }

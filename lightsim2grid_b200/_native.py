@@ -77,7 +77,7 @@ SYMBOLS = ("pf_last_error", "pf_plan_create", "pf_plan_destroy", "pf_plan_info_g
            "pf_flows_device", "pf_flows_host", "pf_ybus_positions", "pf_assemble_ybus_device",
            "pf_set_ybus_values_device", "pf_assemble_sbus_device", "pf_dc_plan_create", "pf_server_create",
            "pf_server_submit", "pf_server_poll", "pf_server_state", "pf_server_destroy", "pf_fdpf_plan_create", "pf_n1_order",
-           "pf_server_configure", "pf_server_device_loop", "pf_server_latency_split")
+           "pf_server_configure", "pf_server_device_loop", "pf_server_latency_split", "pf_host_ybus_route")
 
 
 def load(path=None):
@@ -190,6 +190,8 @@ def load(path=None):
     lib.pf_host_jacobian_pattern.restype = ctypes.c_int
     lib.pf_host_jacobian_pattern.argtypes = [ctypes.c_int, i32p, i32p, f64p, i32p, ctypes.c_int, f64p, i32p,
                                              ctypes.c_int, i32p, ctypes.c_int, ctypes.c_int, i32p, i32p, i32p]
+    lib.pf_host_ybus_route.restype = ctypes.c_int
+    lib.pf_host_ybus_route.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_ulonglong]
     lib.pf_host_schedule_solve.restype = ctypes.c_int
     lib.pf_host_schedule_solve.argtypes = [ctypes.c_int, i32p, i32p, f64p, f64p, f64p, i32p, ctypes.c_int, f64p,
                                            i32p, ctypes.c_int, i32p, ctypes.c_int, ctypes.c_int, f64p, f64p,

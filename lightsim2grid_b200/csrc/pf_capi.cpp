@@ -131,6 +131,22 @@ int check_plan_device(int plan_device, const char *who) {
     return 0;
 }
 
+// Makes `device` current for a scope (no call when it is already).
+struct DeviceGuard {
+    int old = -1;
+    cudaError_t status;
+    explicit DeviceGuard(int device) {
+        status = cudaGetDevice(&old);
+        if (status == cudaSuccess && old == device) old = -1;
+        else if (status == cudaSuccess) status = cudaSetDevice(device);
+    }
+    ~DeviceGuard() {
+        if (old >= 0) cudaSetDevice(old);
+    }
+    DeviceGuard(const DeviceGuard &) = delete;
+    DeviceGuard &operator=(const DeviceGuard &) = delete;
+};
+
 double now() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
@@ -1586,6 +1602,9 @@ int pf_plan_info_get(const pf_plan *pl, pf_plan_info *info) {
 
 int pf_set_ybus_values(pf_plan *pl, const double *ybus_ri) {
     if (!pl || !ybus_ri) return fail(-1, "pf_set_ybus_values: null argument");
+    // the row slots are filled by a kernel, which runs on the plan's device whichever one is current
+    DeviceGuard on(pl->device);
+    if (on.status != cudaSuccess) return cuda_fail(on.status, "pf_set_ybus_values");
     l2g::Plan &P = pl->P;
     const cplx *y = reinterpret_cast<const cplx *>(ybus_ri);
     for (int p = 0; p < P.nnzY; ++p) {
@@ -2599,11 +2618,37 @@ int pf_assemble_ybus_device(int nnz, const int *cptr, const int *cids, const dou
     return e == cudaSuccess ? 0 : cuda_fail(e, "pf_assemble_ybus_device: kernel");
 }
 
+// 0: the kernel reads the source in place.  1: the source is copied into the plan first, as a copy takes any
+// pointer and alignment and the kernel reads 16-byte values of its own device.  2: the stream is another
+// device's, on which the copy runs but the plan's kernel cannot.
+int pf_host_ybus_route(int plan_device, int stream_device, int source_device, unsigned long long source) {
+    if (stream_device != plan_device) return 2;
+    return source_device != plan_device || source % 16 != 0 ? 1 : 0;
+}
+
 int pf_set_ybus_values_device(pf_plan *pl, const double *ybus_ri, void *stream) {
     if (!pl || !ybus_ri) return fail(-1, "pf_set_ybus_values_device: null argument");
-    cudaError_t e = l2g::launch_set_ybus(pl->dp, reinterpret_cast<const double2 *>(ybus_ri), pl->num_sms,
-                                         static_cast<cudaStream_t>(stream));
-    return e == cudaSuccess ? 0 : cuda_fail(e, "pf_set_ybus_values_device");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const char *who = "pf_set_ybus_values_device";
+    int sdev = -1;
+    cudaError_t e = st ? cudaStreamGetDevice(st, &sdev) : cudaGetDevice(&sdev);
+    if (e != cudaSuccess) return cuda_fail(e, who);
+    cudaPointerAttributes at{};
+    if ((e = cudaPointerGetAttributes(&at, ybus_ri)) != cudaSuccess) return cuda_fail(e, who);
+    const int route = pf_host_ybus_route(pl->device, sdev, at.type == cudaMemoryTypeDevice ? at.device : -1,
+                                         reinterpret_cast<uintptr_t>(ybus_ri));
+    double2 *Rx = const_cast<double2 *>(pl->dp.Rx);
+    if (route != 0 && (e = cudaMemcpyAsync(Rx, ybus_ri, (size_t)pl->P.nnzY * sizeof(double2), cudaMemcpyDeviceToDevice,
+                                           st)) != cudaSuccess)
+        return cuda_fail(e, who);
+    // another device's stream: the call waits for the copy and for the kernel
+    if (route == 2 && (e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, who);
+    DeviceGuard on(pl->device);
+    if (on.status != cudaSuccess) return cuda_fail(on.status, who);
+    cudaStream_t run = route == 2 ? nullptr : st;
+    e = l2g::launch_set_ybus(pl->dp, route == 0 ? reinterpret_cast<const double2 *>(ybus_ri) : Rx, pl->num_sms, run);
+    if (e == cudaSuccess && route == 2) e = cudaStreamSynchronize(run);
+    return e == cudaSuccess ? 0 : cuda_fail(e, who);
 }
 
 int pf_assemble_sbus_device(const pf_sbus_layout *lay, int nsteps, const double *gen_p, const double *sgen_p,
