@@ -15,12 +15,16 @@ __device__ __forceinline__ double cabs2(double2 a) { return sqrt(a.x * a.x + a.y
 
 constexpr double kPi = 3.141592653589793;
 
-// t = conj(y V_c) V_r of a Ybus entry (r, c) from b = y V_c: its complex power at the row.  A zero
-// V_c has no dS/d|V|: t becomes NaN, so that the step ends the instance with InifiniteValue.
+// Stands for t of an entry whose V_c is zero (hi word of a NaN that no operation gives).
+constexpr int kZeroVoltage = 0x7ff8a5a5;
+
+// t = conj(y V_c) V_r of a Ybus entry (r, c) from b = y V_c: its complex power at the row.  A V_c whose
+// |V_c|^2 underflows to zero has no dS/d|V|: t is the mark that dsbus reads.
 __device__ __forceinline__ double2 entry_power(double2 b, double2 vc, double2 vr) {
-    const int any = ((__double2hiint(vc.x) | __double2hiint(vc.y)) << 1) | __double2loint(vc.x) | __double2loint(vc.y);
+    const unsigned hi = (unsigned)(__double2hiint(vc.x) | __double2hiint(vc.y)) & 0x7fffffffu;
     const double2 t = cmul(cconj(b), vr);
-    return any != 0 ? t : make_double2(nan(""), nan(""));
+    const double mark = __hiloint2double(kZeroVoltage, 0);
+    return hi >= 0x1e500000u ? t : make_double2(mark, mark);  // either part at least 2^-538
 }
 
 // Jacobian values of Ybus entry (r, c) from t = conj(y V_c) V_r: dS/dVa = -j (t - d) and
@@ -28,9 +32,12 @@ __device__ __forceinline__ double2 entry_power(double2 b, double2 vc, double2 vr
 // BaseNRAlgo::_dSbus_dV, BaseNRAlgo.tpp:228-257, the latter's column c times |V_c|: the Newton
 // unknown is dVm / |V|, which the voltage update multiplies by |V|).  The scaled columns need no
 // |V| and no quotient: two complex products per entry in place of three, a square root and a division.
+// A zero V_c gives the reference's dS/dVa = 0 and NaN dS/d|V|: a bus without a magnitude unknown then leaves
+// the Jacobian singular (SolverReFactor), another one may also end in a step that is not finite.
 __device__ __forceinline__ void dsbus(double2 t, double2 d, double &dvar, double &dvai, double2 &dvm) {
-    dvar = t.y - d.y;
-    dvai = d.x - t.x;
+    const bool zero = __double2hiint(t.x) == kZeroVoltage;
+    dvar = zero ? 0.0 : t.y - d.y;
+    dvai = zero ? 0.0 : d.x - t.x;
     dvm = make_double2(t.x + d.x, t.y + d.y);
 }
 

@@ -168,7 +168,7 @@ __device__ __forceinline__ double2 override_value(const Shared &S, unsigned mask
 
 // (Ybus V)[r] of the row in `slot` (bus r, voltage vr, slice sl): the diagonal, then the off-diagonal
 // entries in column order.  KEEP: t = conj(Y V_c) V_r of every entry goes to T / Td, from which the
-// Jacobian fill and the refinement residual take their values (NaN where V_c is zero, see dsbus).
+// Jacobian fill and the refinement residual take their values (a mark where V_c is zero, see dsbus).
 // The entries of a slice are 32 consecutive values per step (rows sorted by length, so a
 // slice has almost no padding), and the loads of four steps are issued together.
 template <bool KEEP>
