@@ -44,9 +44,12 @@ __device__ __forceinline__ void dsbus(double2 t, double2 d, double &dvar, double
 // a / b.  FP64: from the approximate reciprocal instruction, two Newton steps for the reciprocal, the
 // product, and one correction by the exact remainder (Markstein, "IA-64 and Elementary Functions", ch. 8),
 // without the special cases of the division operator (its range checks and their branch): the
-// quotient of finite operands in the normal range (equal to the operator's in 3.2e9 random cases with exponents
-// up to +-500); a zero pivot gives a non-finite value, as
-// the operator does.  The quotient stands in every step of the elimination's serial chain, and the padding
+// operator's quotient for finite operands in the normal range (a divisor whose significand is all ones, for which the
+// reciprocal's last step does not round as the reciprocal, may round a quotient next to a tie the other way).  An
+// infinite divisor gives zero, as the operator does (its reciprocal is zero, and the residuals are formed
+// with a tiny value in its place); so does one above 2^1022 (the operator: at most 2^-1022 |a|).  A zero or
+// subnormal divisor gives a value that is not finite.
+// The quotient stands in every step of the elimination's serial chain, and the padding
 // operations of a warp's phases (0 / 0) took the operator's slow branch: N-1 batches, 118 buses 0.126
 // -> 0.100 ms, 1354 buses 3.14 -> 2.53 ms, 2848 buses FP64 16.9 -> 16.3 ms, DC 1.28 -> 1.09 ms, 6515
 // buses FP64 66.2 -> 62.6 ms.
@@ -55,12 +58,30 @@ __device__ __forceinline__ void dsbus(double2 t, double2 d, double &dvar, double
 __device__ __forceinline__ double lu_div(double a, double b) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+    const int hi = __double2hiint(b);
+    b = __hiloint2double((hi & 0x7fffffff) >= 0x7ff00000 ? 0 : hi, __double2loint(b));
     r = fma(fma(-b, r, 1.0), r, r);
     r = fma(fma(-b, r, 1.0), r, r);
     const double q = a * r;
     return fma(fma(-b, q, a), r, q);
 }
 __device__ __forceinline__ float lu_div(float a, float b) { return __fdividef(a, b); }
+
+// 1 / x for the dense tail's serial chain over the pivots.
+__device__ __forceinline__ float tail_reciprocal(float x) { return __frcp_rn(x); }
+__device__ __forceinline__ double tail_reciprocal(double x) { return 1.0 / x; }
+
+// a / u from the pivot's reciprocal r: one product and one correction by the exact remainder (Markstein, as
+// above), which rounds as the quotient does, without its branch on special operands.  An infinite pivot gives
+// zero, as the operator does; a zero one, or one whose reciprocal overflows, a value that is not finite.
+__device__ __forceinline__ float tail_quotient(float a, float u, float r) {
+    const float q = a * r;
+    return fmaf(fmaf(-q, r != 0.0f ? u : 0.0f, a), r, q);
+}
+__device__ __forceinline__ double tail_quotient(double a, double u, double r) {
+    const double q = a * r;
+    return fma(fma(-q, r != 0.0 ? u : 0.0, a), r, q);
+}
 
 }  // namespace
 }  // namespace l2g

@@ -893,18 +893,6 @@ __device__ __forceinline__ double lds(unsigned a, double v) {
 __device__ __forceinline__ void sts(unsigned a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
 __device__ __forceinline__ void sts(unsigned a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
 
-// a / u from the pivot's reciprocal r: one product and one correction by the exact remainder
-// (Markstein, "IA-64 and Elementary Functions", ch. 8), which rounds as the quotient does, without its
-// branch on special operands
-__device__ __forceinline__ float tail_quotient(float a, float u, float r) {
-    const float q = a * r;
-    return fmaf(fmaf(-q, u, a), r, q);
-}
-__device__ __forceinline__ double tail_quotient(double a, double u, double r) {
-    const double q = a * r;
-    return fma(fma(-q, u, a), r, q);
-}
-
 // Shared memory of a panel: ush, row c = U(c, c ..) of the diagonal block from column 0, zero past its
 // end; lsh, row c = (0, L(c + 1, c), L(c + 2, c), ...), zero past its end; the reciprocal pivots.  So every step of (a) and (b) reads its NB values from the same place of the row, and
 // the solves are loops whose register arrays move down by one value a step: unrolled over all
@@ -924,14 +912,6 @@ struct TailPanel {
         for (int j = 1; j < W; ++j) v[j - 1] = v[j] - f * u[j];
     }
 };
-
-// 1 / x for (a)'s serial chain.  FP32: the hardware's approximate reciprocal and one Newton step (the
-// quotient it serves corrects itself by the exact remainder).
-__device__ __forceinline__ float tail_reciprocal(float x) {
-    const float r = __fdividef(1.0f, x);
-    return fmaf(fmaf(-x, r, 1.0f), r, r);
-}
-__device__ __forceinline__ double tail_reciprocal(double x) { return 1.0 / x; }
 
 // (a) the diagonal block at row and column J (jb steps; past them the identity) to `sm` and back to D, by
 // the whole CTA: a warp per row (R rows each), a lane per column, the values in registers.  Per pivot:
