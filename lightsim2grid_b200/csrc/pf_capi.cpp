@@ -28,9 +28,6 @@ namespace {
 
 thread_local std::string g_err;
 
-// static shared memory of the Newton and DC kernels (Shared, Segment, the loop's job), rounded up
-constexpr size_t kNrStaticSmem = 2304;
-
 int fail(int code, const std::string &msg) {
     g_err = msg;
     return code;
@@ -759,7 +756,7 @@ int configure(pf_plan *pl) {
         // FP64; both factors in every CTA's shared memory when they fit
         pl->precision = 0;
         pl->refine = false;
-        const size_t static_smem = 4096;  // Shared struct and the three staged plans
+        const size_t static_smem = l2g::kFdpfStaticSmem;
         const size_t sm_in = l2g::fdpf_smem_bytes(pl->dsub[0], pl->dsub[1], true);
         const size_t sm_out = l2g::fdpf_smem_bytes(pl->dsub[0], pl->dsub[1], false);
         const bool fits = pl->dsub[0].compact && pl->dsub[1].compact && sm_in + static_smem <= (size_t)optin;
@@ -785,7 +782,7 @@ int configure(pf_plan *pl) {
         return 0;
     }
     const int lub = pl->precision ? 4 : 8, xb = pl->precision ? 4 : 8;
-    const size_t static_smem = kNrStaticSmem;
+    const size_t static_smem = l2g::kNrStaticSmem;
     // the dense tail's staging area: all columns right of a panel when they fit beside the solve vector
     // (an FP64 one: the mixed form's fallback uses the same width), else chunks of at least 64
     if (P.tail_k > 0) {
@@ -1006,7 +1003,7 @@ int launch_into(pf_plan *pl, l2g::BatchArgs a, int precision, cudaStream_t st, u
         size_t slab = l2g::slab_bytes(pl->dp, lub, in);
         int optin = 0;
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, pl->device);
-        if (in && (need + kNrStaticSmem > (size_t)optin || !pl->dp.compact)) {
+        if (in && (need + l2g::kNrStaticSmem > (size_t)optin || !pl->dp.compact)) {
             in = false;
             need = l2g::smem_bytes(pl->dp, lub, lub, false);
             slab = l2g::slab_bytes(pl->dp, lub, false);
@@ -1367,7 +1364,7 @@ int loop_launch(const LoopShape &sh, const Segment &seg0, const DevQueue &q, int
     l2g::BatchArgs a0 = seg0.A;
     a0.phase_cycles = nullptr;
     a0.trace = nullptr;
-    cudaError_t e = l2g::launch_nr_batch(seg0.P, a0, sh.precision, sh.threads, grid, sh.smem,
+    cudaError_t e = l2g::launch_nr_batch(segment_plan(seg0), a0, sh.precision, sh.threads, grid, sh.smem,
                                          static_cast<cudaStream_t>(stream), M);
     if (e != cudaSuccess) return cuda_fail(e, "request loop: kernel");
     return 0;
@@ -2456,7 +2453,7 @@ int pf_multi_launch(pf_multi *mp, void *stream) {
     l2g::BatchArgs a0 = mp->seg0.A;
     a0.phase_cycles = nullptr;
     a0.trace = nullptr;
-    e = l2g::launch_nr_batch(mp->seg0.P, a0, mp->precision, mp->threads, mp->grid, mp->smem, st, mp->M);
+    e = l2g::launch_nr_batch(l2g::segment_plan(mp->seg0), a0, mp->precision, mp->threads, mp->grid, mp->smem, st, mp->M);
     if (e != cudaSuccess) return cuda_fail(e, "pf_multi_launch: kernel");
     return 0;
 }

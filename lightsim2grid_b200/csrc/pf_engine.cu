@@ -35,15 +35,23 @@ struct Shared {
     double red[32];  // block reductions; the dense tail's backward substitution (one panel's values)
     int ired[32];
     unsigned long long pc[kPhaseSlots];  // per-phase SM cycles (thread 0, when profiled)
-    int opos[kMaxOverrides];
+    // the overrides: rows and columns, or (DC kernel) CSR positions, and values
+    union {
+        int orow[kMaxOverrides];
+        int opos[kMaxOverrides];
+    };
+    int ocol[kMaxOverrides];
     double2 oval[kMaxOverrides];
-    int orow[kMaxOverrides], ocol[kMaxOverrides];  // the overrides' rows and columns
     int novr;
     int job;
     int piv_err;
     int job_failed;
     double slack_absorbed;
 };
+
+static_assert(sizeof(Shared) + sizeof(Segment) + sizeof(QueueJob) + 16 <= kNrStaticSmem,
+              "the Newton kernels' static shared memory, alignment included");
+static_assert(sizeof(Shared) + 3 * sizeof(DevPlan) + 16 <= kFdpfStaticSmem, "the fast decoupled kernel's");
 
 // load with acquire semantics at GPU scope: the job ring entries and segments written before the
 // tail (by the host's copies, in stream order) are seen after it
@@ -142,9 +150,8 @@ __device__ __forceinline__ double2 ybus_value(const DevPlan &P, const Shared &S,
 
 // Stages override i of an instance (caller: one thread per override).  A position outside the pattern
 // (pf_ybus_positions gives -1 there) changes no entry.
-__device__ __forceinline__ void stage_override(const DevPlan &P, Shared &S, int i, int pos, double2 val) {
+__device__ __forceinline__ void stage_override(const PlanArrays &P, Shared &S, int i, int pos, double2 val) {
     const bool in = (unsigned)pos < (unsigned)P.nnzY;
-    S.opos[i] = pos;
     S.oval[i] = val;
     S.orow[i] = in ? P.Rrow[pos] : -1;
     S.ocol[i] = in ? P.Rj[pos] : -1;
@@ -172,7 +179,7 @@ __device__ __forceinline__ double2 override_value(const Shared &S, unsigned mask
 // The entries of a slice are 32 consecutive values per step (rows sorted by length, so a
 // slice has almost no padding), and the loads of four steps are issued together.
 template <bool KEEP>
-__device__ __forceinline__ double2 ybus_row(const DevPlan &P, const Shared &S, const double2 *__restrict__ V, int slot,
+__device__ __forceinline__ double2 ybus_row(const PlanArrays &P, const Shared &S, const double2 *__restrict__ V, int slot,
                                             int r, double2 vr, int2 sl, double2 *__restrict__ T,
                                             double2 *__restrict__ Td) {
     const unsigned mask = row_overrides(S, r);
@@ -213,7 +220,7 @@ __device__ __forceinline__ double2 ybus_row(const DevPlan &P, const Shared &S, c
 // thread per CSR row with 16-byte loads 58 bytes apart) and T kept for the fill and the
 // residual (against a second and third gather of both voltages per entry) are what that takes.
 template <typename XT, bool FB>
-__device__ void mismatch(const DevPlan &P, Shared &S, const double2 *__restrict__ V, double2 *__restrict__ T,
+__device__ void mismatch(const PlanArrays &P, Shared &S, const double2 *__restrict__ V, double2 *__restrict__ T,
                          double2 *__restrict__ Td, double2 *__restrict__ Sd, double2 *__restrict__ Fb,
                          const double2 *__restrict__ Sbus, XT *x, double &norm, int &bad) {
     double lmax = 0.0;
@@ -273,7 +280,7 @@ __device__ __forceinline__ void put_entry(LT *lu, int4 t, double2 te, double2 d)
 // ZERO_ALL: the LU region (shared memory) is cleared whole with 16-byte stores before the
 // entries are written, in place of the gather of the fill-in positions.
 template <typename LT, bool ZERO_ALL>
-__device__ void jacobian_fill(const DevPlan &P, const double2 *__restrict__ T, const double2 *__restrict__ Td,
+__device__ void jacobian_fill(const PlanArrays &P, const double2 *__restrict__ T, const double2 *__restrict__ Td,
                               const double2 *__restrict__ Sd, LT *lu) {
     if constexpr (ZERO_ALL) {
         // lu is 4-byte aligned; the head up to the first 16-byte boundary and the tail are scalar
@@ -619,7 +626,7 @@ __device__ __noinline__ void run_pushes_global(const OP *__restrict__ ops, const
 // The packed operations where a kernel variant can run them: an LU in global memory takes those whose
 // placement keeps a value's operations together (null: the int4 ones).
 template <bool LU_SMEM>
-__device__ __forceinline__ const uint2 *packed_ops(const DevPlan &P, const uint2 *cops) {
+__device__ __forceinline__ const uint2 *packed_ops(const PlanArrays &P, const uint2 *cops) {
     return LU_SMEM || P.cops_runs ? cops : nullptr;
 }
 
@@ -658,7 +665,7 @@ __device__ __forceinline__ void run_lu_program(const uint2 *cops, const int4 *op
 // z(k) / U(k, k): the backward program keeps z undivided.  CHECK: a zero pivot also sets
 // S.piv_err (seen by every thread after the closing barrier).
 template <typename LT, typename XT, bool CHECK = false>
-__device__ __forceinline__ void scale_by_pivots(const DevPlan &P, Shared &S, const LT *lu, XT *x) {
+__device__ __forceinline__ void scale_by_pivots(const PlanArrays &P, Shared &S, const LT *lu, XT *x) {
     int zero = 0;
     for (int k = threadIdx.x; k < P.m; k += blockDim.x) {
         const LT d = lu[P.dpos[k]];
@@ -670,7 +677,7 @@ __device__ __forceinline__ void scale_by_pivots(const DevPlan &P, Shared &S, con
 }
 
 template <typename LT>
-__device__ void check_pivots(const DevPlan &P, Shared &S, const LT *lu) {
+__device__ void check_pivots(const PlanArrays &P, Shared &S, const LT *lu) {
     int zero = 0;
     for (int k = threadIdx.x; k < P.m; k += blockDim.x) zero |= lu[P.dpos[k]] == (LT)0;
     if (zero) S.piv_err = 1;
@@ -684,7 +691,7 @@ __device__ void check_pivots(const DevPlan &P, Shared &S, const LT *lu) {
 // column of a distributed slack: one pass over the mismatch's T, the step gathered from shared
 // memory.  Returns max |F - J dx| to every thread (infinity when a value is not finite).
 template <typename XT>
-__device__ double newton_residual(const DevPlan &P, Shared &S, const double2 *__restrict__ T,
+__device__ double newton_residual(const PlanArrays &P, Shared &S, const double2 *__restrict__ T,
                                   const double2 *__restrict__ Td, const double2 *__restrict__ Sd,
                                   const double2 *__restrict__ Fb, const XT *x, XT *__restrict__ rt) {
     const int ns = P.row_slots, bd = blockDim.x;
@@ -761,7 +768,7 @@ __device__ double newton_residual(const DevPlan &P, Shared &S, const double2 *__
 // and Va and only those buses take |V| and arg(V): two FP64 library calls (and their dependent
 // chains) per bus fewer.  The distributed-slack form keeps its own block-wide re-derivation.
 template <typename XT>
-__device__ double voltage_update(const DevPlan &P, double2 *__restrict__ V, double2 *__restrict__ Vs,
+__device__ double voltage_update(const PlanArrays &P, double2 *__restrict__ V, double2 *__restrict__ Vs,
                                            double *__restrict__ Vm, double *__restrict__ Va,
                                            const XT *__restrict__ dx, const XT *x, bool corrected) {
     const int n = P.n;
@@ -1104,7 +1111,7 @@ __device__ __noinline__ void tail_update(LT *D, int k, int J1, int j0, int w, in
 }
 
 template <typename LT>
-__device__ __noinline__ void tail_factor(const DevPlan &P, LT *lu, LT *D, LT *smem) {
+__device__ __noinline__ void tail_factor(const PlanArrays &P, LT *lu, LT *D, LT *smem) {
     constexpr int NB = tail_panel<LT>();
     const int k = P.tail_k, ld = tail_ld(k), W = P.tail_w;
     tail_gather<LT>(P.tail_map, lu, D, k);
@@ -1129,7 +1136,7 @@ __device__ __noinline__ void tail_factor(const DevPlan &P, LT *lu, LT *D, LT *sm
 // shuffles), then every thread updates rows below it.  Warp 0's chain bounds it: the loop runs a fixed 32
 // steps, so that the block's values are read ahead of the shuffles.
 template <typename LT, typename XT>
-__device__ __noinline__ void tail_forward(const DevPlan &P, const LT *D, XT *x, LT *sm) {
+__device__ __noinline__ void tail_forward(const PlanArrays &P, const LT *D, XT *x, LT *sm) {
     const int k = P.tail_k, ld = tail_ld(k), tid = threadIdx.x, bd = blockDim.x;
     XT *xt = x + P.tail_ct;
     for (int J = 0; J < k; J += 32) {
@@ -1176,7 +1183,7 @@ __device__ __noinline__ void tail_forward(const DevPlan &P, const LT *D, XT *x, 
 // in the chain, here and in tail_forward, the 300-chord N-1 batch took 49.9 instead of 48.3 ms mixed and 91.1
 // instead of 88.8 ms in FP64, the same bits.
 template <typename LT, typename XT>
-__device__ __noinline__ void tail_backward(const DevPlan &P, Shared &S, const LT *D, XT *x, LT *sm) {
+__device__ __noinline__ void tail_backward(const PlanArrays &P, Shared &S, const LT *D, XT *x, LT *sm) {
     const int k = P.tail_k, ld = tail_ld(k), tid = threadIdx.x, bd = blockDim.x;
     XT *xt = x + P.tail_ct;
     const int last = ((k - 1) / 32) * 32;
@@ -1229,7 +1236,7 @@ __device__ __noinline__ void tail_backward(const DevPlan &P, Shared &S, const LT
 // The slab's part before the LU: V (16 B per bus), Vm, Va (8 B per bus), Td, Sd (16 B per row
 // slot), T (16 B per off-diagonal slot); FP32 plans also the FP64 mismatch (16 B per row slot), the
 // first step of a refinement and its residual (a value per unknown).
-__host__ __device__ inline size_t bus_slab_bytes(const DevPlan &P, int x_bytes) {
+__host__ __device__ inline size_t bus_slab_bytes(const PlanArrays &P, int x_bytes) {
     size_t b = (size_t)P.n * 32 + (size_t)P.row_slots * 32 + (size_t)P.row_len * 16;
     if (x_bytes == 4) b += (size_t)P.row_slots * 16 + (size_t)P.m * 8;
     return (b + 255) & ~(size_t)255;
@@ -1248,7 +1255,7 @@ struct Layout {
 };
 
 template <typename LT, typename XT, bool LU_SMEM>
-__device__ __forceinline__ Layout<LT, XT> make_layout(const DevPlan &P, const BatchArgs &A, unsigned char *dyn) {
+__device__ __forceinline__ Layout<LT, XT> make_layout(const PlanArrays &P, const BatchArgs &A, unsigned char *dyn) {
     Layout<LT, XT> L;
     const int n = P.n, m = P.m;
     const size_t xbytes = LU_SMEM ? (size_t)P.lu_offset * sizeof(XT) : (((size_t)m * sizeof(XT) + 15) & ~(size_t)15);
@@ -1290,7 +1297,7 @@ __device__ __forceinline__ Layout<LT, XT> make_layout(const DevPlan &P, const Ba
 
 // Phase bounds and widths of the three programs into shared memory (caller synchronises).
 template <typename LT, typename XT>
-__device__ __forceinline__ void stage_tables(const DevPlan &P, const Layout<LT, XT> &L) {
+__device__ __forceinline__ void stage_tables(const PlanArrays &P, const Layout<LT, XT> &L) {
     for (int i = threadIdx.x; i <= P.fac_nph; i += blockDim.x) L.sb_fac[i] = P.fac_base[i];
     for (int i = threadIdx.x; i <= P.bwd_nph; i += blockDim.x) L.sb_bwd[i] = P.bwd_base[i];
     for (int i = threadIdx.x; i <= P.fwd_nph; i += blockDim.x) L.sb_fwd[i] = P.fwd_base[i];
@@ -1336,7 +1343,7 @@ struct Prof {
 // NARROW: the narrow phases of the packed programs run on their few warps (the 512- and
 // 640-thread variants; at 768 threads the registers it takes cost more than it saves).
 template <typename LT, typename XT, bool LU_SMEM, bool REFINE, bool NARROW>
-__device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, Shared &S, unsigned char *dyn, int first, int count, Prof &pr) {
+__device__ __forceinline__ void solve_job(const PlanArrays &P, const BatchArgs &A, Shared &S, unsigned char *dyn, int first, int count, Prof &pr) {
     const int tid = threadIdx.x;
     const int n = P.n, m = P.m;
     const auto lay = [&]() { return make_layout<LT, XT, LU_SMEM>(P, A, dyn); };
@@ -1576,7 +1583,7 @@ __device__ __forceinline__ void solve_job(const DevPlan &P, const BatchArgs &A, 
 // the FP32 LU used (the next job refills it) and the FP64 LU in the CTA's slab.  The same code
 // as a separate FP64 launch (solve_job with FP64 LU in global memory); a function of its own so
 // that its registers do not add to the FP32 path's.
-__device__ __noinline__ void fp64_rerun(const DevPlan &P, const BatchArgs &A, Shared &S, unsigned char *dyn,
+__device__ __noinline__ void fp64_rerun(const PlanArrays &P, const BatchArgs &A, Shared &S, unsigned char *dyn,
                                         int first, int count) {
     const Layout<double, double> L = make_layout<double, double, false>(P, A, dyn);
     stage_tables<double, double>(P, L);
@@ -1752,7 +1759,8 @@ __global__ void __launch_bounds__(512, 1) dc_batch_kernel(const DevPlan P, const
             __syncthreads();
             if (tid < S.novr) {
                 const int k0 = A.ovr_ptr[inst];
-                stage_override(P, S, tid, A.ovr_pos[k0 + tid], A.ovr_val[k0 + tid]);
+                S.opos[tid] = A.ovr_pos[k0 + tid];
+                S.oval[tid] = A.ovr_val[k0 + tid];
             }
             __syncthreads();
             if (S.novr < 0) {

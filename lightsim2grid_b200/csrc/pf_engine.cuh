@@ -18,14 +18,13 @@ struct DevPushes {
 };
 constexpr int kPushAhead = 4;
 
-// Structure arrays of one plan on the device (see pf_plan.hpp for their meaning).
-struct DevPlan {
+// Structure arrays of one plan on the device (see pf_plan.hpp for their meaning): those that the one-CTA
+// Newton kernel reads, which every CTA keeps in shared memory (Segment), then the others.
+struct PlanArrays {
     int n, m, nnzY, nnzLU, distributed;
-    const int *Rp, *Rj, *Rrow;
-    const double2 *Rx;
+    int dc, slack0;        // DC plan (B = Re(Ybus) without the slack) and its slack bus
+    const int *Rj, *Rrow;  // column and row of a CSR position
     const double *w;
-    const int4 *ytarget;   // 4 LU positions per CSR position
-    const int4 *yjpos;     // 4 J positions per CSR position
     // Ybus rows as the one-CTA kernels walk them: slot s is bus row_bus[s] (-1: padding), rows in
     // decreasing number of off-diagonal entries, a warp per slice of 32 slots; the diagonal per slot
     // (dg_*), the off-diagonal entries of slice g at [row_slice[g].x + 32 u + lane], u <
@@ -33,21 +32,20 @@ struct DevPlan {
     int row_slots, row_len;
     const int *row_bus;
     const int2 *row_slice;
-    const int *off_col, *off_pos;  // column, CSR position
+    const int *off_col;
     const double2 *off_val;
     const int4 *off_target;        // LU positions, as ytarget
     const int2 *off_x;             // xVa, xVm of the column
-    const int *dg_pos;
+    const int *dg_pos;             // CSR position (-1: none)
     const double2 *dg_val;
     const int4 *dg_target;
     const int2 *dg_eq, *dg_x;      // xP, xQ and xVa, xVm of the slot's bus
-    const int *row_of_csr;         // per CSR position: off-diagonal slot, or -1 - diagonal slot
     const int *fillpos;
     int nfill;
-    const int *cpos, *cjpos;
+    const int *cpos;
     const double *cval;
     int nconst;
-    const int *xP, *xQ, *xVa, *xVm;
+    const int *xVa, *xVm;
     int xSlack;
     const double *wJ;        // distributed slack: J(P(r), 0) per bus (0 if none)
     // phase programs (see pf_plan.hpp): operations as int4 (x, y, z, w | kind << 28) and
@@ -67,7 +65,22 @@ struct DevPlan {
     int nar_first[3];   // program k's operation index of the first staged operation (base[nar_a])
     int nar_off[4];     // staged operations of program k at [nar_off[k], nar_off[k + 1])
     const int *dpos;         // pivot position per column (m)
-    int dc, slack0;          // DC plan (B = Re(Ybus) without the slack) and its slack bus
+    // dense tail (global-memory LU plans): steps [tail_ct, tail_ct + tail_k) factorised and
+    // substituted as one dense row-major block in the CTA's slab; tail_map: LU position of each
+    // block entry (-1 outside the pattern)
+    int tail_ct, tail_k;
+    int tail_w;              // columns of U that its staging area holds (a multiple of 32)
+    const int *tail_map;
+};
+struct DevPlan : PlanArrays {
+    const int *Rp;
+    const double2 *Rx;
+    const int4 *ytarget;     // 4 LU positions per CSR position
+    const int4 *yjpos;       // 4 J positions per CSR position
+    const int *off_pos;      // CSR position of an off-diagonal slot
+    const int *row_of_csr;   // per CSR position: off-diagonal slot, or -1 - diagonal slot
+    const int *cjpos;
+    const int *xP, *xQ;
     const double *luval;     // constant factor values (LU layout) of a fast-decoupled system
     DevPushes push[2];       // ... its forward and backward programs over them
     const double *dval;      // ... its pivots (m)
@@ -75,12 +88,6 @@ struct DevPlan {
     // operations (kind 7 padding) and, per phase, the first chunk and the number of rounds
     const int4 *tfac_ops, *tbwd_ops, *tfwd_ops;
     const int *tfac_phase, *tbwd_phase, *tfwd_phase;
-    // dense tail (global-memory LU plans): steps [tail_ct, tail_ct + tail_k) factorised and
-    // substituted as one dense row-major block in the CTA's slab; tail_map: LU position of each
-    // block entry (-1 outside the pattern)
-    int tail_ct, tail_k;
-    int tail_w;              // columns of U that its staging area holds (a multiple of 32)
-    const int *tail_map;
 };
 
 // One batch launch.
@@ -139,9 +146,15 @@ __device__ __forceinline__ double2 *out_row(const BatchArgs &A, int inst, int n)
 
 // One segment of a launch over several plans: a plan and its batch (device memory).
 struct alignas(16) Segment {
-    DevPlan P;
+    PlanArrays P;
     BatchArgs A;
 };
+// The plan argument of a launch whose CTAs take their plans from segments.
+inline DevPlan segment_plan(const Segment &s) {
+    DevPlan P{};
+    static_cast<PlanArrays &>(P) = s.P;
+    return P;
+}
 
 // Launch over several plans (segments): job j runs instances [job_first[j], job_first[j] +
 // job_count[j]) of segment job_seg[j].  segs == nullptr: a launch of one plan.
@@ -181,6 +194,11 @@ struct MultiArgs {
 constexpr int kPhaseSlots = 8;
 
 constexpr int kMaxOverrides = 32;
+
+// Static shared memory set aside beside the dynamic part when a plan is placed: the Newton and DC kernels'
+// (Shared, Segment and the request loop's job) and the fast decoupled kernel's (Shared and three plans).
+// Their size decides which plans are taken: pf_engine.cu asserts that they hold.
+constexpr size_t kNrStaticSmem = 2048, kFdpfStaticSmem = 4096;
 
 // Bytes of the per-CTA global slab and of the dynamic shared memory.
 size_t slab_bytes(const DevPlan &P, int lu_bytes, bool lu_in_smem);
