@@ -192,6 +192,7 @@ struct pf_plan {
     l2g::DevPlan dp{};
     // fast-decoupled plans: the B' and B'' systems
     l2g::DevPlan dsub[2]{};
+    DevBuf push_rows[4];  // fast decoupled: rows of the two systems' forward and backward substitutions
     void *d_sub_int[2] = {nullptr, nullptr}, *d_sub_dbl[2] = {nullptr, nullptr};
     // batch-interleaved kernel: per-CTA slabs, hand-off lists and a row of ones (allocated on
     // first use)
@@ -500,7 +501,7 @@ void build_row_slots(const l2g::Plan &P, RowSlots &R) {
 // Uploads the structure arrays of one plan (and, for a fast-decoupled system, its factor
 // values) into two device blobs and points the fields of `d` into them.
 int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl, const std::vector<double> *luval,
-                int lu_offset = -1, bool compact_ok = true, int threads = 0) {
+                int lu_offset = -1, bool compact_ok = true) {
     std::vector<unsigned char> bi, bd;
     size_t oRp = push(bi, P.Rp), oRj = push(bi, P.Rj), oRrow = push(bi, P.Rrow);
     size_t oyt = push(bi, P.ytarget), oyj = push(bi, P.yjpos);
@@ -564,19 +565,9 @@ int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl,
     size_t oov = push(bd, off), odv = push(bd, dg);
     size_t oRx = push(bd, rx), ow = push(bd, P.weights), ocv = push(bd, P.cval), owJ = push(bd, wJ);
     size_t olu = push(bd, luval ? *luval : std::vector<double>());
-    PushRows push_rows[2];
     std::vector<double> dval;
-    if (luval) {
-        build_push_rows(P.forward, *luval, P.m, threads, push_rows[0]);
-        build_push_rows(P.backward, *luval, P.m, threads, push_rows[1]);
+    if (luval)
         for (int k = 0; k < P.m; ++k) dval.push_back((*luval)[P.dpos[k]]);
-    }
-    size_t opi[2], opm[2], opc[2];
-    for (int k = 0; k < 2; ++k) {
-        opi[k] = push(bi, push_rows[k].idx);
-        opm[k] = push(bi, push_rows[k].mask);
-        opc[k] = push(bd, push_rows[k].coef);
-    }
     size_t odval = push(bd, dval);
     if (d_int) cudaFree(d_int);
     if (d_dbl) cudaFree(d_dbl);
@@ -657,9 +648,6 @@ int upload_plan(const l2g::Plan &P, l2g::DevPlan &d, void *&d_int, void *&d_dbl,
     d.dc = P.dc ? 1 : 0;
     d.slack0 = P.slack0;
     d.luval = luval ? D(olu) : nullptr;
-    for (int k = 0; k < 2; ++k)
-        d.push[k] = l2g::DevPushes{reinterpret_cast<const unsigned *>(bI + opi[k]),
-                                   reinterpret_cast<const unsigned *>(bI + opm[k]), D(opc[k]), push_rows[k].rows};
     d.dval = D(odval);
     const bool tiled = !P.dc && !P.fdpf;
     d.tfac_ops = tiled ? I4(otfo) : nullptr;
@@ -727,8 +715,31 @@ int upload(pf_plan *pl) {
     l2g::fdpf_lu_offsets(pl->P, off[0], off[1], fits);
     for (int k = 0; k < 2; ++k) {
         rc = upload_plan(pl->P.sub[k], pl->dsub[k], pl->d_sub_int[k], pl->d_sub_dbl[k], &pl->P.sublu[k], off[k],
-                         fits, pl->threads);
+                         fits);
         if (rc) return rc;
+    }
+    return 0;
+}
+
+// The padded rows of both systems' substitutions, which the fast decoupled kernel runs when the factors stay in
+// global memory (after configure(), which places them).
+int upload_push_rows(pf_plan *pl) {
+    for (int k = 0; k < 2; ++k) {
+        const l2g::Plan &P = pl->P.sub[k];
+        for (int h = 0; h < 2; ++h) {
+            PushRows R;
+            build_push_rows(h == 0 ? P.forward : P.backward, pl->P.sublu[k], P.m, pl->threads, R);
+            std::vector<unsigned char> b;
+            const size_t oc = push(b, R.coef), oi = push(b, R.idx), om = push(b, R.mask);
+            DevBuf &d = pl->push_rows[2 * k + h];
+            cudaError_t e = d.ensure(b.size());
+            if (e == cudaSuccess) e = cudaMemcpy(d.p, b.data(), b.size(), cudaMemcpyHostToDevice);
+            if (e != cudaSuccess) return cuda_fail(e, "pf_fdpf_plan_create: substitution rows");
+            const unsigned char *at = static_cast<const unsigned char *>(d.p);
+            pl->dsub[k].push[h] = l2g::DevPushes{reinterpret_cast<const unsigned *>(at + oi),
+                                                 reinterpret_cast<const unsigned *>(at + om),
+                                                 reinterpret_cast<const double *>(at + oc), R.rows};
+        }
     }
     return 0;
 }
@@ -837,6 +848,7 @@ void release(pf_plan *pl) {
                       &pl->jfirst, &pl->jcount, &pl->Vout, &pl->iters, &pl->errs, &pl->Jout, &pl->Vlast, &pl->cycles,
                       &pl->Vcase, &pl->casemap})
         b->release();
+    for (DevBuf &b : pl->push_rows) b.release();
     pl->solo.release();
     if (pl->solo_host) cudaFreeHost(pl->solo_host);
     pl->solo_host = nullptr;
@@ -1390,6 +1402,7 @@ int finish_plan(pf_plan *pl, pf_plan **out) {
     cudaEventCreate(&pl->ev1);
     int rc = upload(pl);
     if (!rc) rc = configure(pl);
+    if (!rc && pl->P.fdpf && !pl->lu_in_smem) rc = upload_push_rows(pl);
     if (rc) {
         std::string keep = g_err;
         release(pl);

@@ -1849,7 +1849,8 @@ __global__ void __launch_bounds__(512, 1) dc_batch_kernel(const DevPlan P, const
 // x | LU(B') | LU(B''), each system's packed operations addressing its LU at its lu_offset.
 struct FdpfLayout {
     double *x[2];         // the shared solve vector (both entries equal)
-    const double *lu[2];  // factor values (shared or global)
+    // factors in shared memory: their values, and the programs' phase bounds and widths
+    const double *lu[2];
     int *sbf[2], *swf[2], *sbb[2], *swb[2];
     double2 *V, *T;       // voltages, exp(j Va) of the last P half-step
     double *Vm, *Va;
@@ -1870,18 +1871,20 @@ __device__ __forceinline__ FdpfLayout fdpf_layout(const DevPlan &P, const DevPla
     double *x = reinterpret_cast<double *>(dyn);
     for (int k = 0; k < 2; ++k) {
         L.x[k] = x;
-        L.lu[k] = LU_SMEM ? x + B[k].lu_offset : B[k].luval;
+        L.lu[k] = LU_SMEM ? x + B[k].lu_offset : nullptr;
     }
-    int *t = reinterpret_cast<int *>(dyn + fdpf_region_bytes(B[0], B[1], LU_SMEM));
-    for (int k = 0; k < 2; ++k) {
-        L.sbf[k] = t;
-        t += B[k].fwd_nph + 1;
-        L.sbb[k] = t;
-        t += B[k].bwd_nph + 1;
-        L.swf[k] = t;
-        t += B[k].fwd_nph;
-        L.swb[k] = t;
-        t += B[k].bwd_nph;
+    if constexpr (LU_SMEM) {
+        int *t = reinterpret_cast<int *>(dyn + fdpf_region_bytes(B[0], B[1], true));
+        for (int k = 0; k < 2; ++k) {
+            L.sbf[k] = t;
+            t += B[k].fwd_nph + 1;
+            L.sbb[k] = t;
+            t += B[k].bwd_nph + 1;
+            L.swf[k] = t;
+            t += B[k].fwd_nph;
+            L.swb[k] = t;
+            t += B[k].bwd_nph;
+        }
     }
     unsigned char *slab = A.scratch + (size_t)blockIdx.x * (size_t)A.slab_bytes;
     L.V = reinterpret_cast<double2 *>(slab);
@@ -1898,7 +1901,7 @@ __device__ __forceinline__ FdpfLayout fdpf_layout(const DevPlan &P, const DevPla
 // multiply-add; reading both factors and dividing (16-byte operations, a scattered load of each
 // factor, the quotient's chain) N-1 batches took 68.1 ms (2,848 buses, BX) against 27.8 ms now, 1,354 buses
 // 13.2 -> 8.5 ms, 118 buses 1.40 -> 0.51 ms.
-__device__ __forceinline__ void run_pushes(const DevPushes &R, double *v) {
+__device__ __forceinline__ void run_pushes(const DevPushes R, double *v) {
     constexpr int A = kPushAhead;
     const unsigned *pi = R.idx + threadIdx.x;
     const double *pc = R.coef + threadIdx.x;
@@ -2005,14 +2008,15 @@ __global__ void __launch_bounds__(MAXT, MINB) fdpf_batch_kernel(const DevPlan P0
     {
         for (int k = 0; k < 2; ++k) {
             const DevPlan &b = B[k];
-            for (int i = tid; i <= b.fwd_nph; i += blockDim.x) L.sbf[k][i] = b.fwd_base[i];
-            for (int i = tid; i <= b.bwd_nph; i += blockDim.x) L.sbb[k][i] = b.bwd_base[i];
-            for (int i = tid; i < b.fwd_nph; i += blockDim.x) L.swf[k][i] = b.fwd_width[i];
-            for (int i = tid; i < b.bwd_nph; i += blockDim.x) L.swb[k][i] = b.bwd_width[i];
-            if (LU_SMEM)
+            if constexpr (LU_SMEM) {
+                for (int i = tid; i <= b.fwd_nph; i += blockDim.x) L.sbf[k][i] = b.fwd_base[i];
+                for (int i = tid; i <= b.bwd_nph; i += blockDim.x) L.sbb[k][i] = b.bwd_base[i];
+                for (int i = tid; i < b.fwd_nph; i += blockDim.x) L.swf[k][i] = b.fwd_width[i];
+                for (int i = tid; i < b.bwd_nph; i += blockDim.x) L.swb[k][i] = b.bwd_width[i];
                 for (int i = tid; i < b.nnzLU; i += blockDim.x) L.x[k][b.lu_offset + i] = b.luval[i];
-            else if (tid == 0)
+            } else if (tid == 0) {
                 L.x[k][b.m] = 0.0;  // the padding operations' element (later any value of the other system)
+            }
         }
     }
     __syncthreads();
@@ -2346,6 +2350,7 @@ cudaError_t launch_fdpf_batch(const DevPlan &P, const DevPlan &B0, const DevPlan
 
 size_t fdpf_smem_bytes(const DevPlan &B0, const DevPlan &B1, bool lu_in_smem) {
     size_t b = fdpf_region_bytes(B0, B1, lu_in_smem);
+    if (!lu_in_smem) return b;
     for (const DevPlan *B : {&B0, &B1}) b += (size_t)(2 * (B->fwd_nph + B->bwd_nph) + 2) * sizeof(int);
     return (b + 15) & ~(size_t)15;
 }
