@@ -959,13 +959,18 @@ int analyze_lu(Plan &P, const std::vector<double> &Jx, const PlanOptions &opt, s
     for (int k = 0; k < m; ++k)
         for (int i : Lrows[k]) lrows[i].push_back(k);
 
-    // refactorisation levels: a pivot is applied once every pivot updating its column is done
+    // refactorisation levels: a pivot c is applied once every pivot updating its column or, right of it, its row
+    // is done, so that L(., c) and U(c, .) are final: no operation of a level then reads a value that another one
+    // of it writes.  The row condition follows from the column's where the LU pattern is symmetric; it is not
+    // with several slack buses, one-sided Ybus entries or pivots off the diagonal.
     std::vector<int> level(m, 0);
     P.flops_refactor = 0;
     int nlev = 0;
     for (int k = 0; k < m; ++k) {
         int lv = 0;
         for (int c : Ucols[k]) lv = std::max(lv, level[c] + 1);
+        for (int c : lrows[k])
+            if (!urows[c].empty() && urows[c].back().first > k) lv = std::max(lv, level[c] + 1);
         level[k] = lv;
         nlev = std::max(nlev, lv + 1);
         for (int c : Ucols[k]) P.flops_refactor += P.lcount[c];
