@@ -1060,28 +1060,26 @@ __device__ __noinline__ void tail_solves(LT *D, int k, int J, int j0, int rows, 
 }
 
 // (c): rows and columns right of the panel (M rows from J1, w columns from j0) minus As Bs.  A warp per
-// 4 x 8 register tiles, a tile's columns in groups of 4 that are 32 apart (the lanes of a row read 128
-// consecutive bytes of Bs; columns past the block's last fall in the row padding, their values
-// are never read as entries).
+// 4 x 8 register tiles of TR x 4 values (the lanes of a row read 128 consecutive bytes of Bs; columns past the
+// block's last fall in the row padding, their values are never read as entries).
 template <typename LT>
 __device__ __noinline__ void tail_update(LT *D, int k, int J1, int j0, int w, int W, unsigned sm) {
     constexpr int NB = tail_panel<LT>(), N = Vec16<LT>::N, E = (int)sizeof(LT);
-    constexpr int TR = E == 4 ? 8 : 4, TG = 1;  // register tile: TR rows, TG groups of 4 columns
+    constexpr int TR = E == 4 ? 8 : 4;
     const int ld = tail_ld(k), lda = tail_lda(k), M = k - J1;
     const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const unsigned as = sm + TailPanel<LT>::kBytes, bs = as + (unsigned)(NB * lda * E);
-    const int sr = (M + 4 * TR - 1) / (4 * TR), sc = (w + 32 * TG - 1) / (32 * TG);
+    const int sr = (M + 4 * TR - 1) / (4 * TR), sc = (w + 31) / 32;
     for (int t = threadIdx.x >> 5; t < sr * sc; t += nwarps) {
-        const int ti = t / sc, i0 = (ti * 4 + (lane >> 3)) * TR, q0 = (t - ti * sc) * 32 * TG + (lane & 7) * 4;
+        const int ti = t / sc, i0 = (ti * 4 + (lane >> 3)) * TR, q0 = (t - ti * sc) * 32 + (lane & 7) * 4;
         if (i0 >= M || q0 >= w) continue;
         LT *C = D + (size_t)(J1 + i0) * ld + j0 + q0;
-        LT acc[TR][4 * TG];
+        LT acc[TR][4];
 #pragma unroll
         for (int r = 0; r < TR; ++r)
 #pragma unroll
-            for (int q = 0; q < 4 * TG; q += N) {
-                if (i0 + r < M && q0 + (q >> 2) * 32 < w)
-                    Vec16<LT>::ld(C + (size_t)r * ld + (q >> 2) * 32 + (q & 3), &acc[r][q]);
+            for (int q = 0; q < 4; q += N) {
+                if (i0 + r < M) Vec16<LT>::ld(C + (size_t)r * ld + q, &acc[r][q]);
                 else
 #pragma unroll
                     for (int i = 0; i < N; ++i) acc[r][q + i] = (LT)0;
@@ -1089,23 +1087,21 @@ __device__ __noinline__ void tail_update(LT *D, int k, int J1, int j0, int w, in
         const unsigned pa = as + (unsigned)(i0 * E), pb = bs + (unsigned)(q0 * E);
 #pragma unroll 4
         for (int c = 0; c < NB; ++c) {
-            LT av[TR], bv[4 * TG];
+            LT av[TR], bv[4];
 #pragma unroll
             for (int r = 0; r < TR; r += N) Vec16<LT>::lds(pa + (unsigned)((c * lda + r) * E), av + r);
 #pragma unroll
-            for (int q = 0; q < 4 * TG; q += N)
-                Vec16<LT>::lds(pb + (unsigned)((c * W + (q >> 2) * 32 + (q & 3)) * E), bv + q);
+            for (int q = 0; q < 4; q += N) Vec16<LT>::lds(pb + (unsigned)((c * W + q) * E), bv + q);
 #pragma unroll
             for (int r = 0; r < TR; ++r)
 #pragma unroll
-                for (int q = 0; q < 4 * TG; ++q) acc[r][q] -= av[r] * bv[q];
+                for (int q = 0; q < 4; ++q) acc[r][q] -= av[r] * bv[q];
         }
 #pragma unroll
         for (int r = 0; r < TR; ++r)
 #pragma unroll
-            for (int q = 0; q < 4 * TG; q += N)
-                if (i0 + r < M && q0 + (q >> 2) * 32 < w)
-                    Vec16<LT>::st(C + (size_t)r * ld + (q >> 2) * 32 + (q & 3), &acc[r][q]);
+            for (int q = 0; q < 4; q += N)
+                if (i0 + r < M) Vec16<LT>::st(C + (size_t)r * ld + q, &acc[r][q]);
     }
     __syncthreads();
 }
