@@ -240,7 +240,7 @@ int pf_batch_device(pf_plan *plan, const pf_device_batch *batch, void *stream);
    per-CTA working memory does not fit is rejected with an error, otherwise the launch uses as
    many CTAs as fit.  Mixed form: an instance that does not converge in FP32 is solved again in
    FP64 inside the launch, as pf_batch_device does (the slabs then hold an FP64 LU too, so large
-   plans run on fewer CTAs: about 50 for the 2,848-bus mixed plan).  The current device must be
+   plans run on fewer CTAs: about 48 for the 2,848-bus mixed plan).  The current device must be
    the plan's (else -1, nothing launched).  The first call on a device looks the array's address
    up (cudaGetSymbolAddress) -- make it before any stream capture.  The array is shared by all
    calls and keeps the previous call's contents; the job counter is cleared before each launch.

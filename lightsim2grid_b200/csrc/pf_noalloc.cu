@@ -22,7 +22,7 @@
 //     with an error; otherwise the launch uses as many CTAs as there are slabs in the array
 //     (at most the plan's own grid), so large grids may run on fewer CTAs than
 //     pf_batch_device would use (the 2,848-bus mixed plan, whose slab carries room for the
-//     FP64 fallback's LU, runs on about 50 CTAs).
+//     FP64 fallback's LU, runs on about 48 CTAs).
 //   * The current device must be the plan's device (checked before anything else).
 //   * The first call on a device looks the array's device address up (cudaGetSymbolAddress
 //     with that device current) and caches it; make that first call before any stream
