@@ -318,7 +318,8 @@ int pf_flows_host(const pf_branch_set *br, int n, int nrows, const double *V_ri,
    pf_set_ybus_values_device copies such values (the plan's storage order) into the plan's
    device Ybus, asynchronously: later launches on the plan use them.  The values may be any device
    memory (8-byte aligned) and the stream any device's; with another device's stream than the plan's the
-   call returns when the values are in place.  The plan's host-side
+   call returns when the values are in place.  Captured in a graph, it takes a stream of the plan's device, which is
+   then current.  The plan's host-side
    values (pf_n1_prepare's islanding check, pf_get_J) keep what pf_plan_create or
    pf_set_ybus_values gave. */
 int pf_ybus_positions(const pf_plan *plan, int ncoef, const int *rows, const int *cols, int *pos);

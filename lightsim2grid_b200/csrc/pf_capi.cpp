@@ -2640,13 +2640,25 @@ int pf_set_ybus_values_device(pf_plan *pl, const double *ybus_ri, void *stream) 
     if (!pl || !ybus_ri) return fail(-1, "pf_set_ybus_values_device: null argument");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const char *who = "pf_set_ybus_values_device";
-    int sdev = -1;
-    cudaError_t e = st ? cudaStreamGetDevice(st, &sdev) : cudaGetDevice(&sdev);
+    // The queries are not allowed on a capturing stream (there the stream is taken for one of the current device and
+    // the source is copied), nor, without the relaxed mode, while another stream of the process captures.
+    int sdev = -1, source = -1;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaGetDevice(&sdev);
+    if (e == cudaSuccess && st) e = cudaStreamIsCapturing(st, &capture);
+    if (e == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaPointerAttributes at{};
+        e = cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e == cudaSuccess && st) e = cudaStreamGetDevice(st, &sdev);
+        if (e == cudaSuccess) e = cudaPointerGetAttributes(&at, ybus_ri);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (at.type == cudaMemoryTypeDevice) source = at.device;
+    }
     if (e != cudaSuccess) return cuda_fail(e, who);
-    cudaPointerAttributes at{};
-    if ((e = cudaPointerGetAttributes(&at, ybus_ri)) != cudaSuccess) return cuda_fail(e, who);
-    const int route = pf_host_ybus_route(pl->device, sdev, at.type == cudaMemoryTypeDevice ? at.device : -1,
-                                         reinterpret_cast<uintptr_t>(ybus_ri));
+    const int route = pf_host_ybus_route(pl->device, sdev, source, reinterpret_cast<uintptr_t>(ybus_ri));
+    if (route == 2 && capture != cudaStreamCaptureStatusNone)
+        return fail(-1, "pf_set_ybus_values_device: a capture needs a stream of the plan's device, current");
     double2 *Rx = const_cast<double2 *>(pl->dp.Rx);
     if (route != 0 && (e = cudaMemcpyAsync(Rx, ybus_ri, (size_t)pl->P.nnzY * sizeof(double2), cudaMemcpyDeviceToDevice,
                                            st)) != cudaSuccess)
