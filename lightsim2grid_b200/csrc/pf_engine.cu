@@ -837,7 +837,7 @@ __device__ double voltage_update(const PlanArrays &P, double2 *__restrict__ V, d
 // With the whole panel factorised in shared memory, a barrier per pivot and 5 reads per 16
 // multiply-adds, the 391-step block took 1.64M SM cycles in FP32; now 0.93M: gather 145k, (a) 185k,
 // (b) 200k, (c) 400k (its multiply-adds alone: 156k).  2,848-bus grid with 300 chords, N-1: mixed
-// 72.8 -> 62.0 ms, FP64 131 -> 109 ms.
+// 72.0 -> 60.1 ms, FP64 131 -> 109 ms.
 // A right part wider than tail_w columns (the staging area's
 // share of shared memory) is solved and applied in chunks.  The block's pivots go back to the
 // LU diagonal, where the pivot scaling and the zero-pivot check read them.
@@ -1896,7 +1896,7 @@ __device__ __forceinline__ FdpfLayout fdpf_layout(const DevPlan &P, const DevPla
 // The factors' quotients are formed once per plan, so an operation is 12 streamed bytes and one
 // multiply-add; reading both factors and dividing (16-byte operations, a scattered load of each
 // factor, the quotient's chain) N-1 batches took 68.1 ms (2,848 buses, BX) against 27.8 ms now, 1,354 buses
-// 13.2 -> 8.5 ms, 118 buses 1.40 -> 0.51 ms.
+// 13.2 -> 8.5 ms, 118 buses 1.40 -> 0.51 ms (this change alone, CUDA events around one launch).
 __device__ __forceinline__ void run_pushes(const DevPushes R, double *v) {
     constexpr int A = kPushAhead;
     const unsigned *pi = R.idx + threadIdx.x;

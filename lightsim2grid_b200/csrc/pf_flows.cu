@@ -21,7 +21,6 @@
 namespace l2g {
 namespace {
 
-
 __device__ __forceinline__ double2 cmulf(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -52,13 +51,14 @@ __device__ __forceinline__ double amps_factor(double sn, double vn) { return sn 
 // One CTA per row (grid-stride over rows); each thread takes every NT-th branch and gathers its two
 // voltages through L1.  Bound by those random 16-byte gathers: the rows in work on an SM have to stay in
 // its L1.  So rows of which six do not fit it (kWideRow) run two CTAs of 1024 threads per SM, smaller ones six
-// of 256 (and 40 registers): 2848 buses, 3776 rows: 188 us with eight CTAs of 256 and two square
-// roots and a division per flow, 138 us with six CTAs and one root, 122 us with the two wide CTAs; 300
-// buses, 4000 rows: 19.9 -> 16.9 us (wide CTAs: 23.3); 1600 and 2000 buses, 4000 rows: six narrow CTAs 84 and
-// 104 us, two wide ones 100 and 114, at 2200 the same.  Few rows are spread over more threads: with at most as
-// many rows as wide CTAs run at once (30 rows of 1200 buses: 16.4 -> 12.3 us), or twice as many where a narrow
-// CTA takes long (320 rows of 2000 buses: 20.5 against 24.6 us).  Two or four rows per CTA (branch data read once
-// for all) and tiles of rows staged in shared memory were slower (127-300 and 143 us).
+// of 256 (and 40 registers).  CUDA events around one launch, buffers flushed from L2, 4,500 rows, six narrow against
+// two wide CTAs: 300 buses 22.5 and 36.9 us, 1600 96 and 113, 2000 120 and 127, 2200 135 and 131, 2848 182
+// and 178, 4500 338 and 268, 6515 473 and 453; the 2848-bus N-1 results (3776 rows, 726 of them islanded):
+// 137 and 143 us, 178 with eight CTAs of 256 and two square roots and a division per flow.
+// Few rows are spread over more threads: with at most as many rows as wide CTAs run at once (30 rows of 1200 buses:
+// 16.4 -> 10.2 us), or twice as many where a narrow CTA takes long (450 rows of 2000 buses: 25.6 -> 24.6 us, 600
+// rows the same).  Two or four rows per CTA (branch data read once for all) and tiles of rows staged in shared memory
+// were slower.
 constexpr size_t kWideRow = 34000, kLongRow = 24000;
 template <int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) branch_flows_kernel(const FlowArgs A) {
